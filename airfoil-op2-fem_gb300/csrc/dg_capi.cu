@@ -702,6 +702,22 @@ int dg_tc_round(long long th, long long tl, int sc, double *out) {
   *out = dg::tc_round(th, tl, sc);
   return 0;
 }
+int dg_roe_pair_flux(double gam, int n, const double *qm, const double *qp, const double *nrm, int *taken,
+                     double *f2) {
+  if (n < 0 || !(gam > 1.0) || (n && (!qm || !qp || !nrm || !taken || !f2))) return fail(DG_ERR_ARG, "bad arguments");
+  dg::Phys P{};
+  P.gam = gam;
+  P.gm1 = gam - 1.0;
+  P.rinf = P.pinf = 1.0;
+  P.derive();
+  for (int k = 0; k < n; k++) {
+    taken[k] = dg::roe_small_jump(qm + 4 * k, qp + 4 * k) ? 1 : 0;
+    for (int j = 0; j < 4; j++) f2[4 * k + j] = 0.0;
+    if (taken[k])
+      dg::roe_flux2_small(qm + 4 * k, qp + 4 * k, nrm[2 * k], nrm[2 * k + 1], P.gm1, dg::ff{P.gm1f, P.gm1l}, f2 + 4 * k);
+  }
+  return 0;
+}
 void dg_set_face_block(int threads) { dg::set_face_block(threads); }
 void dg_set_face_regs64(int on) { dg::set_face_regs64(on); }
 int dg_face_regs64(void) { return dg::face_regs64(); }

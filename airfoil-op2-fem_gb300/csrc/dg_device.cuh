@@ -9,6 +9,8 @@
 #include <cmath>
 #include <cstdint>
 
+#include "dg_roe_ff.cuh"
+
 namespace dg {
 
 struct Phys {
@@ -19,6 +21,7 @@ struct Phys {
   // 1/(gamma-1), and the vortex's density coefficient (gamma-1)/(16 gamma pi^2).
   double cinf, rcinf, tgm1, igam, igm1, kvort;
   float gamf, gm1f;              // gamma, gamma - 1 in single precision (the dt estimate)
+  float gm1l;                    // gamma - 1 less gm1f: with it the pair of roe_flux2_small
   // 2/(gamma-1) is 5 (gamma = 1.4; 5 + 9e-16 after the rounding of gamma - 1 in double): the
   // powers x^(2/(gamma-1)) and x^(1/(gamma-1)) are taken as x^5 and x^2 sqrt(x).
   int pow5;
@@ -26,6 +29,7 @@ struct Phys {
   void derive() {
     gamf = (float)gam;
     gm1f = (float)gm1;
+    gm1l = (float)(gm1 - (double)gm1f);
     cinf = sqrt(gam * pinf / rinf);
     rcinf = 1.0 / cinf;
     tgm1 = 2.0 / gm1;
@@ -107,6 +111,15 @@ __device__ __forceinline__ void roe_flux2(const double qm[4], const double qp[4]
   f2[1] = fma(nx, g1, -ny * g2);
   f2[2] = fma(ny, g1, nx * g2);
   f2[3] = g3;
+}
+
+// The flux of a face node: the pair form where the jump is small, else roe_flux2.  A node's states
+// alone decide, so a node gets the same bits whatever launch, range or batch it is part of; a
+// warp with nodes of both kinds runs both.
+__device__ __forceinline__ void roe_flux2_face(const double qm[4], const double qp[4], const double nx,
+                                               const double ny, const Phys &P, double f2[4]) {
+  if (roe_small_jump(qm, qp)) roe_flux2_small(qm, qp, nx, ny, P.gm1, ff{P.gm1f, P.gm1l}, f2);
+  else roe_flux2(qm, qp, nx, ny, P, f2);
 }
 
 // Isentropic vortex state at (x, y, t): vortex/src/set_ic.h:6-22.

@@ -154,7 +154,8 @@ __device__ __forceinline__ void face_node(const Inst &d, const int stage, const 
   // several times an interior node, and last they would leave a tail on a near-idle GPU.
   const int nbf = d.nB * Nfp;
   const Phys &P = d.P;
-  double qm[4], qp[4], f2[4];
+  double qm[4], qp[4], f2[4], nx, ny, sL, sR = 0.0;
+  double *ol, *orr = nullptr;
   if (tid >= nbf) {
     const int e = (tid - nbf) / Nfp, i = (tid - nbf) - e * Nfp;
     const int4 ed = __ldg(&d.edges[e]);
@@ -162,9 +163,10 @@ __device__ __forceinline__ void face_node(const Inst &d, const int stage, const 
     const int iR = (ed.z >> 4) ? Nfp - 1 - i : i;
     const int nodeL = __ldg(&d.fmask[fL * Nfp + i]), nodeR = __ldg(&d.fmask[fR * Nfp + iR]);
     const double *gl = d.geo + (size_t)cL * 16 + 4 + 3 * fL;
-    const double nx = __ldg(gl), ny = __ldg(gl + 1);
-    const double sL = __ldg(gl + 2);
-    const double sR = -__ldg(d.geo + (size_t)cR * 16 + 4 + 3 * fR + 2);
+    nx = __ldg(gl);
+    ny = __ldg(gl + 1);
+    sL = __ldg(gl + 2);
+    sR = -__ldg(d.geo + (size_t)cR * 16 + 4 + 3 * fR + 2);
     if constexpr (PDL) {
       pdl_wait();
       pdl_trigger();
@@ -174,20 +176,17 @@ __device__ __forceinline__ void face_node(const Inst &d, const int stage, const 
     double2 a = ld2(wl), b = ld2(wl + 2), c = ld2(wr), dd = ld2(wr + 2);
     qm[0] = a.x; qm[1] = a.y; qm[2] = b.x; qm[3] = b.y;
     qp[0] = c.x; qp[1] = c.y; qp[2] = dd.x; qp[3] = dd.y;
-    roe_flux2(qm, qp, nx, ny, P, f2);
-    double *ol = d.flux + (((size_t)cL * 3 + fL) * Nfp + i) * 4;
-    double *orr = d.flux + (((size_t)cR * 3 + fR) * Nfp + iR) * 4;
-    st2(ol, sL * f2[0], sL * f2[1]);
-    st2(ol + 2, sL * f2[2], sL * f2[3]);
-    st2(orr, sR * f2[0], sR * f2[1]);
-    st2(orr + 2, sR * f2[2], sR * f2[3]);
+    ol = d.flux + (((size_t)cL * 3 + fL) * Nfp + i) * 4;
+    orr = d.flux + (((size_t)cR * 3 + fR) * Nfp + iR) * 4;
   } else {
     const int b = tid / Nfp, i = tid - b * Nfp;
     const int4 bd = __ldg(&d.bedges[b]);
     const int c = bd.x, f = bd.y, type = bd.z;
     const int node = __ldg(&d.fmask[f * Nfp + i]);
     const double *g = d.geo + (size_t)c * 16 + 4 + 3 * f;
-    const double nx = __ldg(g), ny = __ldg(g + 1), s = __ldg(g + 2);
+    nx = __ldg(g);
+    ny = __ldg(g + 1);
+    sL = __ldg(g + 2);
     if constexpr (PDL) {
       pdl_wait();
       pdl_trigger();
@@ -203,10 +202,14 @@ __device__ __forceinline__ void face_node(const Inst &d, const int stage, const 
     } else {
       bc_state(type, qm, nx, ny, P, qp);
     }
-    roe_flux2(qm, qp, nx, ny, P, f2);
-    double *o = d.flux + (((size_t)c * 3 + f) * Nfp + i) * 4;
-    st2(o, s * f2[0], s * f2[1]);
-    st2(o + 2, s * f2[2], s * f2[3]);
+    ol = d.flux + (((size_t)c * 3 + f) * Nfp + i) * 4;
+  }
+  roe_flux2_face(qm, qp, nx, ny, P, f2);  // one call for both kinds: its code is long
+  st2(ol, sL * f2[0], sL * f2[1]);
+  st2(ol + 2, sL * f2[2], sL * f2[3]);
+  if (orr) {
+    st2(orr, sR * f2[0], sR * f2[1]);
+    st2(orr + 2, sR * f2[2], sR * f2[3]);
   }
 }
 

@@ -339,6 +339,12 @@ int dg_tc_operator_digits(int N, int *dims, double *S, int *fexp, int *digits);
  * device runs.  *out = (th * 2^32 + tl) * 2^sc rounded to the nearest double, ties to even, for
  * |th| < 2^41, |tl| < 2^49 (the joined level sums) and -1022 <= sc <= 900; DG_ERR_ARG outside. */
 int dg_tc_round(long long th, long long tl, int sc, double *out);
+/* Host-only (no GPU needed): the face kernels' Roe flux for small jumps, the same code the device
+ * runs (its seeds apart).  For n pairs of states qm, qp [n][4] and unit normals nrm [n][2], taken[k]
+ * is 1 where the small-jump form applies (else the general FP64 form runs on the device) and f2
+ * [n][4] receives twice the flux there, 0 elsewhere. */
+int dg_roe_pair_flux(double gam, int n, const double *qm, const double *qp, const double *nrm, int *taken,
+                     double *f2);
 /* Cell ranges of the step graph for solvers whose graph is built from now on: 0 automatic (the
  * default: ranges of at least 128 tiles of 32 cells, at most 4), 1 a single range (the seven
  * launches as one chain), 2..32 that many ranges (fewer if the mesh has fewer tiles). */
