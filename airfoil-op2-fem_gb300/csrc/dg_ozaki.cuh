@@ -94,11 +94,16 @@ __device__ __forceinline__ uint32_t oz_pair(const uint32_t hl, const uint32_t ll
 // bit length of T, at most 1997), so no subnormal or overflow case arises.  The result equals
 // RN(th 2^(32+sc) + tl 2^sc), the sum of the two exact parts rounded once.
 // Host and device alike (the host copy serves the library's rounding check, dg_tc_round).
-__host__ __device__ __forceinline__ int oz_clz64(const unsigned long long x) {
+// Three 32-bit words, whole words and then bits shifted out to the left, ~40 instructions (as a 64-bit
+// form with both signs and shift directions apart: ~70).  With the level sums joined by 32-bit
+// multiplies, the operands aligned by right shifts only and each output's shuffles next to its
+// rounding, steps in runs on O-grids: K = 32768 184.5 -> 180.0 / 295.8 -> 291.7 / 490.4 -> 471.0 us at
+// N = 3 / 4 / 5; K = 131072 683 -> 662 / 1148 -> 1132 / 1901 -> 1831 us (same bits).
+__host__ __device__ __forceinline__ int oz_clz32(const uint32_t x) {
 #ifdef __CUDA_ARCH__
-  return __clzll((long long)x);
+  return __clz((int)x);
 #else
-  return __builtin_clzll(x);
+  return __builtin_clz(x);
 #endif
 }
 __host__ __device__ __forceinline__ double oz_double(const unsigned long long b) {
@@ -111,53 +116,43 @@ __host__ __device__ __forceinline__ double oz_double(const unsigned long long b)
 #endif
 }
 
+__host__ __device__ __forceinline__ uint32_t oz_shl96(const uint32_t hi, const uint32_t lo, const int z) {
+#ifdef __CUDA_ARCH__
+  return __funnelshift_l(lo, hi, z);
+#else
+  return z ? (hi << z) | (lo >> (32 - z)) : hi;
+#endif
+}
+
 __host__ __device__ __forceinline__ double oz_round(const long long th, const long long tl, const int sc) {
-  // T = H 2^32 + L with 0 <= L < 2^32, then |T| = MH 2^32 + ML (MH < 2^42, ML < 2^32)
-  const long long H = th + (tl >> 32);
-  const unsigned long long L = (unsigned long long)tl & 0xFFFFFFFFull;
-  const unsigned long long sign = H < 0 ? 0x8000000000000000ull : 0ull;
-  unsigned long long MH, ML;
-  if (H < 0) {
-    MH = (unsigned long long)(-H) - (L ? 1ull : 0ull);
-    ML = L ? 0x100000000ull - L : 0ull;
-  } else {
-    MH = (unsigned long long)H;
-    ML = L;
+  // |T| as 96 bits a2:a1:a0 (T = H 2^32 + L with 0 <= L < 2^32; negated by complement and increment)
+  const unsigned long long H = (unsigned long long)(th + (tl >> 32));
+  const uint32_t m = (uint32_t)((long long)H >> 63);
+  uint32_t a0 = (uint32_t)tl ^ m, a1 = (uint32_t)H ^ m, a2 = (uint32_t)(H >> 32) ^ m;
+  const unsigned long long lo = (((unsigned long long)a1 << 32) | a0) + (m & 1u);
+  a2 += (lo == 0ull) ? (m & 1u) : 0u;
+  a1 = (uint32_t)(lo >> 32);
+  a0 = (uint32_t)lo;
+  int be = sc + 1117;  // the biased exponent, less one, when bit 31 of a2 leads
+#pragma unroll
+  for (int w = 0; w < 2; w++) {  // whole words: a2 becomes the leading word (0 only for T = 0)
+    const bool z = a2 == 0u;
+    a2 = z ? a1 : a2;
+    a1 = z ? a0 : a1;
+    a0 = z ? 0u : a0;
+    be -= z ? 32 : 0;
   }
-  // the leading bits in one 64-bit word S = |T| / 2^off; below 2^63 exactly (off = 0), else the
-  // 10 dropped bits of ML only decide ties (sticky)
-  unsigned long long S;
-  int off;
-  bool sticky;
-  if (MH >> 31) {
-    S = (MH << 22) | (ML >> 10);
-    off = 10;
-    sticky = (ML & 0x3FFull) != 0ull;
-  } else {
-    S = (MH << 32) | ML;
-    off = 0;
-    sticky = false;
-  }
-  if (S == 0ull) return 0.0;
-  const int nb = 64 - oz_clz64(S);  // bit length of S
-  unsigned long long q;  // significand, 2^52 <= q < 2^53
-  int e2;                // value = q 2^(e2 + sc)
-  if (nb <= 53) {        // (off = 0 here: S >= 2^53 otherwise)
-    q = S << (53 - nb);
-    e2 = nb - 53;
-  } else {
-    const int sh = nb - 53;
-    q = S >> sh;
-    const unsigned long long rem = S & ((1ull << sh) - 1ull), half = 1ull << (sh - 1);
-    if (rem > half || (rem == half && (sticky || (q & 1ull)))) q++;
-    e2 = sh + off;
-    if (q >> 53) {  // rounded up to 2^53
-      q >>= 1;
-      e2++;
-    }
-  }
-  const unsigned long long be = (unsigned long long)(e2 + sc + 52 + 1023);
-  return oz_double(sign | (be << 52) | (q & 0xFFFFFFFFFFFFFull));
+  if (a2 == 0u) return 0.0;
+  const int z = oz_clz32(a2);
+  be -= z;
+  const uint32_t x2 = oz_shl96(a2, a1, z), x1 = oz_shl96(a1, a0, z);
+  const uint32_t sticky = (a0 << z) != 0u ? 1u : 0u;
+  // 53 leading bits, and one more when the 11 bits after them (and the sticky bit) are above half,
+  // or half and the last bit odd; the carry may run into the exponent, as it should
+  const unsigned long long M = (((unsigned long long)x2 << 32) | x1) >> 11;
+  const uint32_t up = ((x1 & 0x7FFu) + 0x3FFu + (((x1 >> 11) & 1u) | sticky)) >> 11;
+  const unsigned long long r = ((unsigned long long)(uint32_t)be << 52) + M + up;
+  return oz_double(r | ((unsigned long long)(m & 0x80000000u) << 32));
 }
 
 // Bit pattern of a double -> its magnitude aligned to the biased column exponent em as an integer,
@@ -167,8 +162,8 @@ template <int SH>
 __device__ __forceinline__ long long oz_align(const unsigned long long b, const int em) {
   const int e = (int)((b >> 52) & 0x7FF);
   const unsigned long long M = e ? ((b & 0xFFFFFFFFFFFFFull) | (1ull << 52)) : 0ull;
-  const int sh = e - em + SH;
-  const unsigned long long m = sh >= 0 ? (M << sh) : (sh > -64 ? (M >> -sh) : 0ull);
+  // e <= em: a right shift of M 2^SH (below 2^56), all of it gone at 63
+  const unsigned long long m = (M << SH) >> min(em - e, 63);
   return (b >> 63) ? -(long long)m : (long long)m;
 }
 
@@ -263,11 +258,13 @@ __device__ __forceinline__ void oz_tile(const double *__restrict__ Xd, double *_
   // C fragment: acc[.][0] (row g, col 2t), [1] (g, 2t+1), [2] (g+8, 2t), [3] (g+8, 2t+1).
   // One output: the level sums lev[] of (row g + 8 r, operator row n) joined and rounded.
   auto finish = [&](const float lev[7], const int n, const int r) {
-    long long l[7];
+    // |lev[L]| <= (L + 1) 32 255^2, so that 256 lev[0] + lev[1] and 256 lev[3] + lev[4] (below 2^31 - 6.3e6)
+    // fit 32 bits
+    int l[7];
 #pragma unroll
-    for (int L = 0; L < 7; L++) l[L] = (long long)__float2int_rz(lev[L]);
-    const long long th = l[0] * 65536LL + l[1] * 256LL + l[2];
-    const long long tl = l[3] * 16777216LL + l[4] * 65536LL + l[5] * 256LL + l[6];
+    for (int L = 0; L < 7; L++) l[L] = __float2int_rz(lev[L]);
+    const long long th = (long long)(l[0] * 256 + l[1]) * 256LL + l[2];
+    const long long tl = (long long)(l[3] * 256 + l[4]) * 65536LL + ((long long)l[5] * 256LL + l[6]);
     const int fe = c_ozf[T][NORD][P][n];
     const int sc = em[r] + fe - 2046 - 62 + (3 - SH);
     double out;
@@ -291,17 +288,17 @@ __device__ __forceinline__ void oz_tile(const double *__restrict__ Xd, double *_
     // lane 3 takes the (row g + 8, column 2t' + 1) output of lanes t' = 0, 1, 2 (their level sums by
     // shuffle), so every lane rounds three outputs instead of three lanes rounding four.  Same
     // values, same rounding.
+    // The shuffles go with each output, not ahead of all three: 14 values fewer live (N = 3 element
+    // kernel at 64 registers).
     const bool hi = t == 3;
-    float x[3][7];
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-#pragma unroll
-      for (int L = 0; L < 7; L++) x[k][L] = __shfl_sync(0xffffffffu, acc[L][3], (lane & ~3) | k);
 #pragma unroll
     for (int k = 0; k < 3; k++) {
       float lev[7];
 #pragma unroll
-      for (int L = 0; L < 7; L++) lev[L] = hi ? x[k][L] : acc[L][k];
+      for (int L = 0; L < 7; L++) {
+        const float x = __shfl_sync(0xffffffffu, acc[L][3], (lane & ~3) | k);
+        lev[L] = hi ? x : acc[L][k];
+      }
       // k = 0, 1: row g, columns 2t, 2t + 1; k = 2: row g + 8, column 2t
       const int n = 8 * NT + (hi ? 2 * k + 1 : 2 * t + (k & 1));
       finish(lev, n, hi || k == 2 ? 1 : 0);
@@ -312,19 +309,17 @@ __device__ __forceinline__ void oz_tile(const double *__restrict__ Xd, double *_
     // on all four lanes of a group with half the outputs each.  Same values, same rounding.
     const bool hi = t >= 2;
     const int src = hi ? lane - 2 : lane;
-    float lv[2][7];
-#pragma unroll
-    for (int L = 0; L < 7; L++)
-#pragma unroll
-      for (int cc = 0; cc < 2; cc++) {
-        const float x = __shfl_sync(0xffffffffu, acc[L][2 + cc], src);
-        lv[cc][L] = hi ? x : acc[L][cc];
-      }
     const int tt = hi ? t - 2 : t, r = hi ? 1 : 0;
 #pragma unroll
     for (int cc = 0; cc < 2; cc++) {
+      float lev[7];
+#pragma unroll
+      for (int L = 0; L < 7; L++) {
+        const float x = __shfl_sync(0xffffffffu, acc[L][2 + cc], src);
+        lev[L] = hi ? x : acc[L][cc];
+      }
       const int n = 8 * NT + 2 * tt + cc;
-      if (n < R) finish(lv[cc], n, r);
+      if (n < R) finish(lev, n, r);
     }
   } else {
 #pragma unroll
