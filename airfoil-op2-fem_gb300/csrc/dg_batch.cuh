@@ -120,28 +120,26 @@ __global__ void __launch_bounds__(32 * np_of(N), elem_min_blocks(N, TC)) batch_e
 // The step's finalize of every instance, with the calc_dt maximum taken from the element
 // kernels' single-precision estimates as dt_finalize_kernel does for one solver: fblocks[b] =
 // {instance k, first estimate of the block, blocks of instance k, 0}; each block's 8 warps read
-// 32 estimates each (one ballot), evaluate the candidates within 1e-4 of the instance's largest
-// estimate in FP64 (each by the whole warp), combine them by atomicMax, and the instance's last
+// kFinalizeEst / 8 estimates, evaluate the candidates within 1e-4 of the instance's largest
+// estimate in FP64 (dt_candidates), combine them by atomicMax, and the instance's last
 // block (the counter in its step state, no waiting) advances its t and sets its dt.  Instances
 // with a frozen dt get one block that advances t.
+constexpr int kFinalizeEst = 1024;  // estimates per block
 __global__ void __launch_bounds__(256) batch_dt_finalize_kernel(const Inst *insts, const int4 *fblocks) {
   const int4 fb = fblocks[blockIdx.x];
   const Inst &d = insts[fb.x];
   unsigned long long best = 0ull;
   if (d.dt_mode == 0) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int Np = np_of(d.N), n = ((d.K + 31) >> 5) * Np;
+    const int n = ((d.K + kDtCells - 1) / kDtCells) * np_of(d.N);
     const float thr = __uint_as_float(d.st->dt_est_max) * 0.9999f;
-    const int base = fb.y + warp * 32;
-    unsigned cand = __ballot_sync(0xffffffffu, base + lane < n && d.dt_est[base + lane] >= thr);
-    while (cand) {
-      const int k = __ffs((int)cand) - 1;
-      cand &= cand - 1u;
-      const int j = base + k, tile = j / Np;
-      unsigned long long v = 0ull;
-      DG_DISPATCH_RT(d.N, (v = dt_node_bits<NN>(d, tile * 32 + lane, j - tile * Np)));
-      best = v > best ? v : best;
+    int j[kFinalizeEst / 256];
+    float est[kFinalizeEst / 256];
+    for (int k = 0; k < kFinalizeEst / 256; k++) {
+      j[k] = fb.y + 256 * k + threadIdx.x;
+      est[k] = j[k] < n ? d.dt_est[j[k]] : -1.0f;
     }
+    for (int k = 0; k < kFinalizeEst / 256; k++)
+      DG_DISPATCH_RT(d.N, (best = dt_candidates<NN>(d, j[k], est[k], thr, best)));
   }
   finalize_block_end(d, best, (unsigned)fb.z);
 }
@@ -225,13 +223,13 @@ struct Batch {
     }
     maxNp = np_of(maxN);
     std::vector<Inst> insts;
-    std::vector<int4> fbs;  // the finalize's blocks: 256 estimates each, one for a frozen dt
+    std::vector<int4> fbs;  // the finalize's blocks: kFinalizeEst estimates each, one for a frozen dt
     for (size_t k = 0; k < solvers.size(); k++) {
       const Inst &d = solvers[k]->d;
       insts.push_back(d);
-      const int n = ((d.K + 31) / 32) * np_of(d.N);
-      const int g = d.dt_mode == 0 ? std::max(1, (n + 255) / 256) : 1;
-      for (int b = 0; b < g; b++) fbs.push_back(make_int4((int)k, 256 * b, g, 0));
+      const int n = ((d.K + kDtCells - 1) / kDtCells) * np_of(d.N);
+      const int g = d.dt_mode == 0 ? std::max(1, (n + kFinalizeEst - 1) / kFinalizeEst) : 1;
+      for (int b = 0; b < g; b++) fbs.push_back(make_int4((int)k, kFinalizeEst * b, g, 0));
     }
     nfb = (int)fbs.size();
     if (cudaMalloc(&d_fblocks, sizeof(int4) * fbs.size()) != cudaSuccess ||

@@ -339,7 +339,8 @@ __device__ __forceinline__ void oz_tile(const double *__restrict__ Xd, double *_
 
 // Parity 0: K0 staged slots from slot 0 to R0 outputs from row 0; parity 1: K1 slots from SLOT1
 // to R1 outputs from YROW1.  Work units: (parity, n-tile of 8 outputs, group of 4 cells); warp w
-// of nw takes units w, w + nw, ...  PRE: the operands come from oz_prep (see oz_tile).
+// of nw takes units w, w + nw, ...  PRE: the operands come from oz_prep (see oz_tile).  G: groups of
+// 4 cells in the tile.
 template <int N, int T, int K0, int R0, int K1, int R1, int SLOT1, int YROW1, int NT, bool PRE, int XST>
 __device__ __forceinline__ void oz_unit(const double *Xd, double *Yd, const int w, const int c0, const int lane,
                                         const int *Ems) {
@@ -356,13 +357,14 @@ __device__ __forceinline__ void oz_unit(const double *Xd, double *Yd, const int 
   }
 }
 
-template <int N, int T, int K0, int R0, int K1, int R1, int SLOT1, int YROW1, bool PRE = false, int XST = 128>
+template <int N, int T, int K0, int R0, int K1, int R1, int SLOT1, int YROW1, bool PRE = false, int XST = 128,
+          int G = 8>
 __device__ __forceinline__ void oz_product(const double *Xd, double *Yd, const int warp, const int nw,
                                            const int lane, const int *Ems = nullptr) {
   constexpr int NTT = (R0 + 7) / 8 + (R1 + 7) / 8;
   static_assert(NTT <= 4, "at most 4 n-tiles");
-  for (int u = warp; u < 8 * NTT; u += nw)
-    oz_unit<N, T, K0, R0, K1, R1, SLOT1, YROW1, 0, PRE, XST>(Xd, Yd, u >> 3, (u & 7) * 4, lane, Ems);
+  for (int u = warp; u < G * NTT; u += nw)
+    oz_unit<N, T, K0, R0, K1, R1, SLOT1, YROW1, 0, PRE, XST>(Xd, Yd, u / G, (u & (G - 1)) * 4, lane, Ems);
 }
 
 // Sign and magnitude of an integer below 2^63 in one 64-bit word (sign in bit 63).
@@ -371,28 +373,30 @@ __device__ __forceinline__ unsigned long long oz_signmag(const long long v) {
 }
 
 // The even/odd butterfly and the operand alignment of the element kernel's contraction, once per
-// staged value, by the first 2 NC threads of the block (two per column of the NC: the slot pairs
-// are dealt alternately, lanes l and l ^ 16 share a column).  Pairs k < NUo: slot k (x_a) and slot NUe + k
+// staged value, by the first TPC NC threads of the block (TPC per column of the NC: the slot pairs
+// are dealt round-robin; lanes 32 / TPC apart share a column).  Pairs k < NUo: slot k (x_a) and slot NUe + k
 // (x_b) become x_a + x_b and x_a - x_b; the unpaired slots NUo <= k < NUe stay single.  Every
 // value is aligned to the largest exponent E of its column's NK = NUe + NUo values as a 55-bit
 // integer (so that sums fit 56 bits), the sums and differences are exact, and each is stored as
 // sign and magnitude in its slot's 64 bits; Ems[column] = E (biased).
-template <int NUe, int NUo, int XST, int NC = 128>
+template <int NUe, int NUo, int XST, int NC = 128, int TPC = 2>
 __device__ __forceinline__ void oz_prep(double *Xd, int *Ems, const int tid) {
-  static_assert(NC % 16 == 0, "columns in groups of 16");
-  if (tid >= 2 * NC) return;
-  const int c = (tid & 15) | ((tid >> 5) << 4), h = (tid >> 4) & 1;
+  constexpr int CPW = 32 / TPC;  // columns per warp
+  static_assert(NC % CPW == 0, "whole warps");
+  if (tid >= TPC * NC) return;
+  const int c = (tid & (CPW - 1)) + (tid >> 5) * CPW, h = (tid & 31) / CPW;
   const uint32_t *Xw = reinterpret_cast<const uint32_t *>(Xd);
   int e = 0;
 #pragma unroll
-  for (int k = h; k < NUe; k += 2) {
+  for (int k = h; k < NUe; k += TPC) {
     e = max(e, (int)((Xw[2 * (k * XST + c) + 1] >> 20) & 0x7FF));
     if (k < NUo) e = max(e, (int)((Xw[2 * ((NUe + k) * XST + c) + 1] >> 20) & 0x7FF));
   }
-  e = max(e, __shfl_xor_sync(0xffffffffu, e, 16));
+#pragma unroll
+  for (int o = CPW; o < 32; o <<= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
   if (h == 0) Ems[c] = e;
 #pragma unroll
-  for (int k = h; k < NUe; k += 2) {
+  for (int k = h; k < NUe; k += TPC) {
     const long long ma = oz_align<2>((unsigned long long)__double_as_longlong(Xd[k * XST + c]), e);
     if (k < NUo) {
       const long long mb = oz_align<2>((unsigned long long)__double_as_longlong(Xd[(NUe + k) * XST + c]), e);
@@ -411,7 +415,25 @@ __device__ __forceinline__ void oz_prep(double *Xd, int *Ems, const int tid) {
 // conflict), with 132 rows t and t + 2 do (2-way; ~1 M conflicts per launch at N = 3), with 130
 // the rows start 8 banks apart and the 16 lanes cover all 32 banks once.  Step 232.3 -> 231.2 us
 // at N = 3 and 379.9 -> 377.7 us at N = 4 (runs of 40 steps; same bits).
-constexpr int kElemSlot = 130;
+constexpr int elem_slot(int cells) { return 4 * cells + 2; }  // (8 and 16 cells: the rows are 8 banks apart too)
+constexpr int kElemSlot = elem_slot(32);
+
+// Small tiles: the orders whose contraction is on the tensor cores, their cells, the threads of a
+// block (one per cell and node, and at least a warp per unit of the contraction) and, of a tile of
+// CT cells, the threads per column of the operand pre-pass.
+constexpr bool elem_small_used(int N) { return N >= 1 && N <= kOzMaxN; }
+constexpr int elem_small_ct(int N) { return N == 2 ? 16 : 8; }
+constexpr int elem_small_units(int N) { return N <= 2 ? 1 : (N == 3 ? 2 : (N == 4 ? 3 : 4)); }  // n-tiles
+constexpr int elem_small_threads(int N) {
+  const int a = (elem_small_ct(N) * ((N + 1) * (N + 2) / 2) + 31) / 32;
+  const int b = elem_small_ct(N) / 4 * elem_small_units(N);
+  return 32 * (a > b ? a : b);
+}
+constexpr int oz_prep_threads(int N, int CT) {
+  if (CT == 32 || N < 3) return 2;
+  const int t = elem_small_threads(N) / (4 * CT);
+  return t >= 8 ? 8 : (t >= 4 ? 4 : 2);
+}
 
 // The element kernel's contraction: Y rows 0..NRe-1 = S_e, Y rows NRe.. = S_o, on the operands
 // oz_prep made from the staged pairs (sums below slot NUe, differences from slot NUe on).  Earlier
@@ -420,18 +442,18 @@ constexpr int kElemSlot = 130;
 // each unit's operands (322 us at N = 3; slower at N = 4, 5, where every n-tile redid the doubled
 // alignment); oz_prep, once per value and spread over 256 threads, gives 294 / 446 / 652 us (with
 // the padded slots, 308.5 / 484 / 736 us before it).
-template <int N, int NUe, int NUo, int NRe, int NRo>
+template <int N, int NUe, int NUo, int NRe, int NRo, int CT = 32>
 __device__ __forceinline__ void oz_contract(const double *Xd, double *Yd, const int warp, const int nw,
                                             const int lane, const int *Ems) {
-  oz_product<N, 0, NUe, NRe, NUo, NRo, NUe, NRe, true, kElemSlot>(Xd, Yd, warp, nw, lane, Ems);
+  oz_product<N, 0, NUe, NRe, NUo, NRo, NUe, NRe, true, elem_slot(CT), CT / 4>(Xd, Yd, warp, nw, lane, Ems);
 }
 
 // The dense form: Y rows 0..NP-1 (one per node) = A (NP x NK) applied to the NK slots in their
 // natural order (Fr, Fs, face points).
-template <int N, int NK, int NP>
+template <int N, int NK, int NP, int CT = 32>
 __device__ __forceinline__ void oz_contract_dense(const double *Xd, double *Yd, const int warp, const int nw,
                                                   const int lane) {
-  oz_product<N, 2, NK, NP, 0, 0, NK, NP, false, kElemSlot>(Xd, Yd, warp, nw, lane);
+  oz_product<N, 2, NK, NP, 0, 0, NK, NP, false, elem_slot(CT), CT / 4>(Xd, Yd, warp, nw, lane);
 }
 
 // The adjoint element kernel's transposed contraction: columns 0..NUe-1 = S_e^T (even rows of the

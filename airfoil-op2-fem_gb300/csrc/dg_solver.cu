@@ -25,7 +25,7 @@
 //                    fscale again as floats in the last 16 bytes (the dt estimate)
 //   edges  int4 {cL, cR, fL | fR << 2 | reverse << 4, 0};  bedges int4 {cell, face, type, 0}
 //   bxy    [nB][Nfp][2] boundary face-node coordinates (vortex boundary)
-//   dt_est [tiles][Np] floats: each node-warp's largest calc_dt estimate of the last stage
+//   dt_est [K / 8][Np] floats: the largest calc_dt estimate of the last stage of a node in 8 cells
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -244,6 +244,10 @@ __device__ __forceinline__ float f32_trunc(const double x) {
   return __uint_as_float(sign | mag);
 }
 
+// Cells whose calc_dt estimates of one node share an entry of Inst::dt_est: the smallest tile of
+// the element kernels, so that every tile size writes whole entries.
+constexpr int kDtCells = 8;
+
 // src/calc_dt.h for one node in FP64: (N+1)^2 / 2 (|v| + c) fs as the bit pattern of a
 // non-negative double (fs the larger fscale of the node's faces).  The element kernel and
 // dt_finalize_kernel evaluate it with the same operations, so either gives the same maximum.
@@ -347,14 +351,12 @@ __device__ __forceinline__ void stage_combine(const Inst &d, const int stage, co
       est = ((N + 1) * (N + 1) * 0.5f) * (sqrtf(v2) + cs) * fsf;
       if (!(est == est) || est > 3.0e38f) est = 3.0e38f;  // non-finite: always a candidate
     }
-    if (active) {
-      float wm = est;
-      for (int o = 16; o > 0; o >>= 1) wm = fmaxf(wm, __shfl_xor_sync(0xffffffffu, wm, o));
-      if (lane == 0) {
-        d.dt_est[(size_t)(e >> 5) * Np + i] = wm;
-        atomicMax(&d.st->dt_est_max, __float_as_uint(wm));  // non-negative: ordered as integers
-      }
-    }
+    // the largest of each 8 cells of one node, and the warp's largest into the step state
+    float wm = est;
+    for (int o = 1; o < kDtCells; o <<= 1) wm = fmaxf(wm, __shfl_xor_sync(0xffffffffu, wm, o));
+    if (live && (threadIdx.x & (kDtCells - 1)) == 0) d.dt_est[(size_t)((unsigned)e / kDtCells) * Np + i] = wm;
+    for (int o = kDtCells; o < 32; o <<= 1) wm = fmaxf(wm, __shfl_xor_sync(0xffffffffu, wm, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(&d.st->dt_est_max, __float_as_uint(wm));  // non-negative: ordered as integers
   }
 }
 
@@ -448,27 +450,31 @@ __global__ void __launch_bounds__(32 * np_of(N)) elem_kernel(const Inst d, const
 // TC: 0 the even/odd contraction in FP64, 1 the even/odd blocks on the tensor cores (N = 3-5; the
 // butterfly and the operand alignment by oz_prep), 2 the dense rows on the tensor cores at N = 1, 2
 // (no butterfly) and form 1 at N = 3-5.
-template <int N, bool PDL = false, int TC = 0>
-__device__ __forceinline__ void elem_tile_sym(const Inst &d, const int stage, const int e0, const int lane,
-                                              const int i, double2 *X) {
+// CT: cells of the tile (32, or 8 or 16 for the tensor-core forms); lane and warp are the thread's
+// place in the block, thread t = 32 warp + lane takes cell t % CT and node t / CT.
+template <int N, bool PDL = false, int TC = 0, int CT = 32>
+__device__ __forceinline__ void elem_tile_sym(const Inst &d, const int stage, const int e0, const int wlane,
+                                              const int warp, double2 *X) {
   constexpr int Np = np_of(N), Nfp = N + 1, NK = nk_of(N);
   constexpr int NUe = Sym<N>::NUe, NUo = Sym<N>::NUo, NRe = Sym<N>::NRe;
   constexpr int NPin = NUo;  // input pairs
-  constexpr int kS2 = kElemSlot / 2;  // double2 per staged slot
+  constexpr int kS = elem_slot(CT), kS2 = kS / 2;  // doubles and double2 per staged slot
   constexpr bool DENSE = ozd_used(N, TC);           // dense rows, slots in natural order
   constexpr bool SYMTC = !DENSE && oz_used(N, TC != 0);  // even/odd blocks on the tensor cores
   double2 *Y = X + NK * kS2;
   int *Ems = reinterpret_cast<int *>(Y + Np * kS2);  // column exponents of the prepared operands
-  const int nthr = 32 * Np, tid = i * 32 + lane;
+  static_assert(CT == 32 || DENSE || SYMTC, "small tiles: tensor-core forms only");
+  const int nthr = CT * Np, tid = warp * 32 + wlane;
+  const int lane = CT == 32 ? wlane : tid & (CT - 1), i = CT == 32 ? warp : (int)((unsigned)tid / CT);  // cell, node
   const bool active = i < Np;
   const int e = e0 + lane;
   const bool live = active && e < d.K;
   const Phys &P = d.P;
   // the tile's face fluxes (contiguous in HBM) go straight into their slots by asynchronous
-  // copies: j = tid + m*nthr, so the face point f = j / 32 is uniform in a warp
+  // copies: j = tid + m*nthr, so at CT = 32 the face point f = j / 32 is uniform in a warp
   auto stage_face_fluxes = [&]() {
-    for (int j = active ? tid : 3 * Nfp * 32; j < 3 * Nfp * 32; j += nthr) {
-      const int f = j >> 5, el = j & 31;
+    for (int j = active ? tid : 3 * Nfp * CT; j < 3 * Nfp * CT; j += nthr) {
+      const int f = (int)((unsigned)j / CT), el = j & (CT - 1);
       const bool ok = e0 + el < d.K;
       const double *fp = d.flux + (((size_t)(ok ? e0 + el : 0)) * 3 * Nfp + f) * 4;
       const int pf = DENSE ? 2 * Np + f : c_pos[N][2 * Np + f];
@@ -524,7 +530,7 @@ __device__ __forceinline__ void elem_tile_sym(const Inst &d, const int stage, co
   __syncthreads();
   if constexpr (SYMTC) {
     // the butterfly in integers and the operand alignment, once per value
-    oz_prep<NUe, NUo, kElemSlot>(reinterpret_cast<double *>(X), Ems, tid);
+    oz_prep<NUe, NUo, kS, 4 * CT, oz_prep_threads(N, CT)>(reinterpret_cast<double *>(X), Ems, tid);
     __syncthreads();
   } else if constexpr (!DENSE) {
     // butterfly over the input pairs: slot p <- x_a + x_b, slot NUe + p <- x_a - x_b (the
@@ -543,13 +549,13 @@ __device__ __forceinline__ void elem_tile_sym(const Inst &d, const int stage, co
   double r0 = 0.0, r1 = 0.0, r2 = 0.0, r3 = 0.0;
   if constexpr (DENSE) {
     // the dense rows on the tensor cores: Y row i is node i's right-hand side
-    oz_contract_dense<N, NK, Np>(reinterpret_cast<const double *>(X), reinterpret_cast<double *>(Y), i,
-                                 (int)(blockDim.x * blockDim.y) >> 5, lane);
+    oz_contract_dense<N, NK, Np, CT>(reinterpret_cast<const double *>(X), reinterpret_cast<double *>(Y), warp,
+                                     (int)(blockDim.x * blockDim.y) >> 5, wlane);
   } else if constexpr (SYMTC) {
     // the contraction on the tensor cores (dg_ozaki.cuh), every warp of the block taking part
-    oz_contract<N, NUe, NUo, NRe, Sym<N>::NRo>(reinterpret_cast<const double *>(X),
-                                                     reinterpret_cast<double *>(Y), i,
-                                                     (int)(blockDim.x * blockDim.y) >> 5, lane, Ems);
+    oz_contract<N, NUe, NUo, NRe, Sym<N>::NRo, CT>(reinterpret_cast<const double *>(X),
+                                                   reinterpret_cast<double *>(Y), warp,
+                                                   (int)(blockDim.x * blockDim.y) >> 5, wlane, Ems);
   } else if (!active) {
   } else if (i < NRe) {
 #pragma unroll
@@ -605,15 +611,15 @@ __device__ __forceinline__ void elem_tile_sym(const Inst &d, const int stage, co
       w[0] = a.x; w[1] = a.y; w[2] = b.x; w[3] = b.y;
     }
   }
-  stage_combine<N>(d, stage, e, active, live, i, lane, w, r0, r1, r2, r3);
+  stage_combine<N>(d, stage, e, active, live, i, wlane, w, r0, r1, r2, r3);
   // X and Y are rewritten by the next tile only after every warp is past this point
   __syncthreads();
 }
 
 // Dynamic shared memory of the even/odd element kernels: NK staged slots, Np output rows and the
-// 128 column exponents of the prepared tensor-core operands.
-constexpr size_t elem_sym_smem(int N) {
-  return (size_t)(nk_of(N) + np_of(N)) * kElemSlot * sizeof(double) + 128 * sizeof(int);
+// column exponents (4 per cell) of the prepared tensor-core operands.
+constexpr size_t elem_sym_smem(int N, int CT = 32) {
+  return (size_t)(nk_of(N) + np_of(N)) * elem_slot(CT) * sizeof(double) + 4 * CT * sizeof(int);
 }
 
 // MB: minimum resident blocks per SM the register allocation must allow (oz_min_blocks for the
@@ -627,6 +633,20 @@ __global__ void __launch_bounds__(32 * np_of(N), MB) elem_kernel_sym(const Inst 
   extern __shared__ double2 Xs[];  // [NK][32] x 4 doubles, then [Np][32] x 4 doubles
   pdl_trigger();  // the next face kernel may be scheduled (it waits for this grid's writes)
   elem_tile_sym<N, PW, TC>(d, stage, (tile0 + (int)blockIdx.x) * 32, threadIdx.x, threadIdx.y, Xs);
+}
+
+// The same over tiles of elem_small_ct(N) cells (tensor-core forms, TC = 2; used as elem_small says):
+// elem_small_threads threads, of which CT Np hold a cell's node and every warp takes part in the
+// operand pre-pass and the contraction.  Compiled for 24 or 28 warps per SM, which at 128 to 256
+// threads a block leaves 72 to 80 registers a thread (one block per SM: up to 127 registers and
+// fewer warps, K = 32768 N = 5 515 against 472 us per step; N = 2 at 24 / 28 warps 119.8 / 115.4 us).
+template <int N, bool PW>
+__global__ void __launch_bounds__(elem_small_threads(N), (N <= 3 ? 28 : 24) * 32 / elem_small_threads(N))
+    elem_kernel_small(const Inst d, const int stage, const int tile0) {
+  constexpr int CT = elem_small_ct(N);
+  extern __shared__ double2 Xs[];
+  pdl_trigger();
+  elem_tile_sym<N, PW, 2, CT>(d, stage, (tile0 + (int)blockIdx.x) * CT, threadIdx.x & 31, threadIdx.x >> 5, Xs);
 }
 
 #include "dg_elem_ws.cuh"
@@ -704,28 +724,61 @@ __device__ __forceinline__ void finalize_block_end(const Inst &d, unsigned long 
   }
 }
 
+// The candidates among 32 estimates, est this lane's, the one at index j (0 past the last): those at
+// or above thr are evaluated four at a time, a quarter of the warp (8 lanes, one per cell) each.
+template <int N>
+__device__ __forceinline__ unsigned long long dt_candidates(const Inst &d, const int j, const float est, const float thr,
+                                                            unsigned long long best) {
+  constexpr int Np = np_of(N);
+  const int lane = threadIdx.x & 31;
+  unsigned cand = __ballot_sync(0xffffffffu, est >= thr);
+  while (cand) {
+    int mine = -1;
+#pragma unroll
+    for (int q = 0; q < 32 / kDtCells; q++) {
+      const int k = __ffs((int)cand) - 1;  // -1 when none is left
+      if (lane / kDtCells == q) mine = k;
+      cand &= cand - 1u;
+    }
+    const int jm = __shfl_sync(0xffffffffu, j, mine < 0 ? lane : mine);
+    if (mine >= 0) {
+      const int grp = jm / Np;
+      const unsigned long long v = dt_node_bits<N>(d, grp * kDtCells + (lane & (kDtCells - 1)), jm - grp * Np);
+      best = v > best ? v : best;
+    }
+  }
+  return best;
+}
+
+// Warp w of the grid's G takes sectors of 8 estimates w, w + G, w + 2G, ...: neighbouring estimates
+// (candidates cluster where the cells are smallest) go to different warps, four sectors per load
+// instruction, four loads in flight.
 template <int N>
 __global__ void __launch_bounds__(256) dt_finalize_kernel(const Inst d) {
-  constexpr int Np = np_of(N);
+  constexpr int U = 4;
   pdl_wait();
   pdl_trigger();
-  const int n = ((d.K + 31) >> 5) * Np;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int n = ((d.K + kDtCells - 1) / kDtCells) * np_of(N);
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, gs = gridDim.x * nw;
   const float thr = __uint_as_float(d.st->dt_est_max) * 0.9999f;
-  // warp w of the grid takes the estimates w, w + G, w + 2G, ... (G warps in the grid): its lanes
-  // read 32 of them at once, and the candidates among them are evaluated one after the other,
-  // each by the whole warp (lane = cell of the tile)
   unsigned long long best = 0ull;
-  const int gs = gridDim.x * nw;
-  for (int base = blockIdx.x * nw + warp; base < n; base += 32 * gs) {
-    const int jl = base + lane * gs;
-    unsigned cand = __ballot_sync(0xffffffffu, jl < n && d.dt_est[jl] >= thr);
-    while (cand) {
-      const int k = __ffs((int)cand) - 1;
-      cand &= cand - 1u;
-      const int j = base + k * gs, tile = j / Np;
-      const unsigned long long v = dt_node_bits<N>(d, tile * 32 + lane, j - tile * Np);
-      best = v > best ? v : best;
+  for (int s0 = blockIdx.x * nw + (threadIdx.x >> 5); 8 * s0 < n; s0 += 4 * U * gs) {
+    int j[U];
+    float est[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      j[u] = 8 * (s0 + (4 * u + (lane >> 3)) * gs) + (lane & 7);
+      est[u] = j[u] < n ? d.dt_est[j[u]] : -1.0f;
+    }
+    bool any = false;
+#pragma unroll
+    for (int u = 0; u < U; u++) any |= est[u] >= thr;
+    if (!__any_sync(0xffffffffu, any)) continue;
+#pragma unroll 1
+    for (int u = 0; u < U; u++) {  // one copy of the FP64 evaluation's code
+      const int ju = u == 0 ? j[0] : (u == 1 ? j[1] : (u == 2 ? j[2] : j[3]));
+      const float eu = u == 0 ? est[0] : (u == 1 ? est[1] : (u == 2 ? est[2] : est[3]));
+      best = dt_candidates<N>(d, ju, eu, thr, best);
     }
   }
   finalize_block_end(d, best, gridDim.x);
@@ -1014,11 +1067,52 @@ static void elem_ws_launch(const Inst &d, int stage, int t0, int t1, cudaStream_
     elem_kernel_ws<N, false><<<grid, ws_threads(N), smem, s>>>(d, stage, t0, t1);
 }
 
+// Whether a mesh of K cells takes the small tiles (elem_small_ct(N) cells per block) instead of 32-cell
+// tiles: the same bits either way.  A 32-cell tile's phases follow one another for ~25k clocks
+// even alone on an SM, whose FP64 pipe its node-warps share while other SMs idle; small tiles
+// spread the same work over more SMs and, on ~80 registers instead of 64, spill nothing.  On large
+// meshes the 32-cell blocks' shared operator fragments and face blocks between them win at N = 1, 3
+// and 4.  Steps in runs, 32-cell / small tiles (O-grids, GB300):
+//   N = 1: K = 3072 58.2 / 48.4, 28000 84.5 / 81.5, 73728 144 / 160 us
+//   N = 2: 2048 57.4 / 55.9, 32768 131.0 / 115.4, 262144 896 / 788 us
+//   N = 3: 2048 70.9 / 55.7, 8192 85.7 / 77.7, 14000 111.9 / 103.6, 28000 162.9 / 163.9 us
+//   N = 4: 1152 86.2 / 63.8, 8192 114.2 / 112.7, 9600 115.9 / 118.8, 28000 255.7 / 275.9 us
+//   N = 5: 1152 74.9 / 64.6, 3072 88.1 / 96.9, 6000 157.8 / 138.1, 9600 165.9 / 179.2,
+//          28000 423.7 / 410.3, 262144 3784 / 3714 us
+// (N = 5 keeps 32 cells where their blocks, one per SM, nearly fill one or two waves).
+static bool elem_small(int N, int K) {
+  switch (N) {
+    case 1: return K <= 32768;
+    case 2: return true;
+    case 3: return K <= 20480;
+    case 4: return K <= 8192;
+    case 5: return !((K > 16 * 152 && K <= 32 * 152) || (K > 8192 && K <= 64 * 152));
+    default: return false;
+  }
+}
+
+template <int N>
+static void elem_small_launch(const Inst &d, int stage, int c0, int c1, cudaStream_t s, bool attr) {
+  constexpr int CT = elem_small_ct(N), threads = elem_small_threads(N);
+  const int t0 = c0 / CT, t1 = (std::min(c1, d.K) + CT - 1) / CT;
+  const size_t smem = elem_sym_smem(N, CT);
+  if (attr && pdl_on())
+    launch_pdl(elem_kernel_small<N, true>, dim3(t1 - t0), dim3(threads), smem, s, d, stage, t0);
+  else if (attr)
+    launch_pdl(elem_kernel_small<N, false>, dim3(t1 - t0), dim3(threads), smem, s, d, stage, t0);
+  else
+    elem_kernel_small<N, false><<<t1 - t0, threads, smem, s>>>(d, stage, t0);
+}
+
 // Element tiles [t0, t1) of one stage in the current form (the even/odd forms; form 0, dense FP64,
 // only as a whole-mesh launch with attr).
 template <int N>
 static void launch_elem_form(const Inst &d, int stage, int t0, int t1, cudaStream_t s, bool attr) {
   if (t1 <= t0) return;
+  if constexpr (elem_small_used(N)) {
+    if (g_elem_variant == 3 && !g_elem_ws && elem_small(N, d.K))
+      return elem_small_launch<N>(d, stage, 32 * t0, 32 * t1, s, attr);
+  }
   if constexpr (ws_used(N)) {
     if (g_elem_ws && g_elem_variant >= 2) return elem_ws_launch<N>(d, stage, t0, t1, s, attr);
   }
@@ -1080,6 +1174,12 @@ static cudaError_t set_smem_attr() {
   if constexpr (N == 3) both(elem_kernel_sym<N, 1, 2, true>, elem_kernel_sym<N, 1, 2, false>);
   if constexpr (ozd_used(N, 2))
     both(elem_kernel_sym<N, 2, oz_min_blocks(N), true>, elem_kernel_sym<N, 2, oz_min_blocks(N), false>);
+  if constexpr (elem_small_used(N)) {
+    for (auto k : {elem_kernel_small<N, true>, elem_kernel_small<N, false>})
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)elem_sym_smem(N, elem_small_ct(N)));
+  }
   if constexpr (ws_used(N)) {
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(elem_kernel_ws<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ws_smem(N));
@@ -1403,7 +1503,7 @@ int Solver::create(const Config &c, const Mesh &m, std::string &err) {
   int *fm = (int *)dalloc(sizeof(int) * 3 * Nfp);
   d.fmask = fm;
   d.st = (StepState *)dalloc(sizeof(StepState));
-  d.dt_est = (float *)dalloc((size_t)((K + 31) / 32) * Np * sizeof(float));
+  d.dt_est = (float *)dalloc((size_t)((K + kDtCells - 1) / kDtCells) * Np * sizeof(float));
   {
     int dev = 0;
     CK(cudaGetDevice(&dev));
@@ -1462,9 +1562,9 @@ void Solver::enqueue_step(cudaStream_t s) {
 
 void Solver::enqueue_finalize(cudaStream_t s, bool pdl) {
   if (d.dt_mode == 0 && d.dt_est) {
-    // one block per SM at most, at least 8 estimates per block
-    const int n = ((K + 31) / 32) * np_of(cfg.N);
-    const int g = std::max(1, std::min(sm_count > 0 ? sm_count : 1, (n + 7) / 8));
+    // one block per SM at most, at least 32 estimates per block
+    const int n = ((K + kDtCells - 1) / kDtCells) * np_of(cfg.N);
+    const int g = std::max(1, std::min(sm_count > 0 ? sm_count : 1, (n + 31) / 32));
     DG_DISPATCH(cfg.N, pdl ? launch_pdl(dt_finalize_kernel<NN>, dim3(g), dim3(256), 0, s, d)
                            : (dt_finalize_kernel<NN><<<g, 256, 0, s>>>(d), void()));
   } else if (pdl) {

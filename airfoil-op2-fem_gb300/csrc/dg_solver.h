@@ -47,8 +47,7 @@ struct Inst {
   StepState *st;
   double *dt_hist;
   unsigned long long dt_hist_len;
-  // Per 32-cell tile and node, the largest single-precision calc_dt estimate of the node-warp
-  // ([tiles][Np]), written by the last stage's element kernel when non-null: the FP64 maximum is
+  // Per 8 cells and node, the largest single-precision calc_dt estimate ([K / 8][Np]), written by the last stage's element kernel when non-null: the FP64 maximum is
   // then taken over the candidates by dt_finalize_kernel.  Null: the element kernel takes it.
   float *dt_est;
   Phys P;
