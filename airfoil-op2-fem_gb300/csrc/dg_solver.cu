@@ -1587,28 +1587,31 @@ void Solver::enqueue_step_events(cudaStream_t s, cudaEvent_t *ev) {
   cudaEventRecord(ev[7], s);
 }
 
+// The cell ranges of this solver's step graphs and the steps in one of them (once, and again after
+// drop_graphs).
 int Solver::build_graph(std::string &err) {
-  if (graph_exec) return 0;
+  if (parts) return 0;
   const int P = g_elem_variant ? step_parts_for(K) : 1;  // the dense FP64 form has no tile ranges
   if (P > 1) {
     if (int rc = build_parts(P, err)) return rc;
   } else {
     parts = 1;
   }
+  graph_steps = steps_per_graph();
+  return 0;
+}
+
+// G steps as one graph; captured when a run first needs it.
+int Solver::capture_steps(int G, cudaGraph_t &gr, cudaGraphExec_t &ex, std::string &err) {
+  if (ex) return 0;
   const unsigned long long flags = (parts > 1 && (step_graph_flags() & 6)) ? cudaGraphInstantiateFlagUseNodePriority : 0;
-  // one step, and (over cell ranges) graph_steps steps in one graph
-  graph_steps = parts > 1 ? steps_per_graph() : 1;
-  for (int k = 0; k < (graph_steps > 1 ? 2 : 1); k++) {
-    const int G = k == 0 ? 1 : graph_steps;
-    cudaGraph_t &gr = k == 0 ? graph : graphG;
-    cudaGraphExec_t &ex = k == 0 ? graph_exec : graphG_exec;
-    CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    if (parts > 1) enqueue_step_parts(stream, nullptr, nullptr, G);
-    else enqueue_step(stream);
-    cudaError_t ce = cudaStreamEndCapture(stream, &gr);
-    if (ce != cudaSuccess) { err = std::string("graph capture: ") + cudaGetErrorString(ce); return -6; }
-    CK(cudaGraphInstantiate(&ex, gr, flags));
-  }
+  CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+  if (parts > 1) enqueue_step_parts(stream, nullptr, nullptr, G);
+  else
+    for (int g = 0; g < G; g++) enqueue_step(stream);
+  cudaError_t ce = cudaStreamEndCapture(stream, &gr);
+  if (ce != cudaSuccess) { err = std::string("graph capture: ") + cudaGetErrorString(ce); return -6; }
+  CK(cudaGraphInstantiate(&ex, gr, flags));
   return 0;
 }
 
@@ -1644,9 +1647,12 @@ int step_parts_for(int K) {
   return std::max(1, std::min(4, T / 128));
 }
 
-// Steps in one launch of the step graph over cell ranges (run() launches it as often as it fits,
-// then the one-step graph for the rest).  On the K = 32768 O-grid at N = 3, 40 steps in one run():
-// 254.3 / 245.9 / 241.6 / 239.4 us per step with 1 / 2 / 4 / 8 steps per graph.
+// Steps in one launch of the step graph (run() launches it as often as it fits, then the one-step
+// graph for the rest).  Steps in runs with 1 / 2 / 4 / 8 steps per graph, over cell ranges (the next
+// step's face launches overlap the last element launches): K = 32768, N = 3 204.5 / 195.4 / 190.1 /
+// 186.9 us; one chain of launches (fewer graph launches, whose gaps a short step feels): K = 2048
+// 58.1 / 53.3 / 51.3 / 50.5 us at N = 3, 54.8 / 50.1 / 45.5 / 45.5 at N = 2, 64.8 / 60.9 / 59.7 / 59.4
+// at N = 4.
 static std::atomic<int> g_steps_per_graph{8};
 void set_steps_per_graph(int g) { g_steps_per_graph = (g >= 1 && g <= 8) ? g : 8; }
 int steps_per_graph() { return g_steps_per_graph; }
@@ -1923,8 +1929,12 @@ int Solver::step(int nsteps, bool use_graph, std::string &err) {
   if (use_graph) {
     if (int rc = build_graph(err)) return rc;
     int i = 0;
-    if (graph_steps > 1 && graphG_exec)
+    if (graph_steps > 1 && nsteps >= graph_steps) {
+      if (int rc = capture_steps(graph_steps, graphG, graphG_exec, err)) return rc;
       for (; i + graph_steps <= nsteps; i += graph_steps) CK(cudaGraphLaunch(graphG_exec, stream));
+    }
+    if (i < nsteps)
+      if (int rc = capture_steps(1, graph, graph_exec, err)) return rc;
     for (; i < nsteps; i++) CK(cudaGraphLaunch(graph_exec, stream));
   } else {
     for (int i = 0; i < nsteps; i++) enqueue_step(stream);

@@ -95,7 +95,7 @@ void set_pdl(int on);
 // graphs built from now on.
 constexpr int kMaxStepParts = 32;
 void set_step_parts(int p);
-// Steps per launch of the step graph over cell ranges (1..8, default 8).
+// Steps per launch of the step graph (1..8, default 8).
 void set_steps_per_graph(int g);
 int steps_per_graph();
 // Tuning of that graph: bit 0 no programmatic dependent launch between its kernels, bit 1
@@ -128,6 +128,7 @@ struct Solver {
   int sm_count = 0;
   void enqueue_step_events(cudaStream_t s, cudaEvent_t *ev);
   int build_graph(std::string &err);
+  int capture_steps(int G, cudaGraph_t &gr, cudaGraphExec_t &ex, std::string &err);
   // The step graph as a DAG of cell ranges (build_graph with more than one range).
   std::vector<int4> h_edges, h_bedges;  // device edge records in mesh order (host copy)
   int parts = 0;                         // ranges of the graph built (0: none yet)
@@ -140,7 +141,7 @@ struct Solver {
   // One step of the ranges' DAG on s; with q_in, the input is uploaded range by range first, with
   // q_out the result is downloaded range by range (host buffers, pinned).
   void enqueue_step_parts(cudaStream_t s, const double *q_in = nullptr, double *q_out = nullptr, int nsteps = 1);
-  cudaGraph_t graphG = nullptr;  // graph_steps steps in one graph (over cell ranges)
+  cudaGraph_t graphG = nullptr;  // graph_steps steps in one graph
   cudaGraphExec_t graphG_exec = nullptr;
   int graph_steps = 1;
   int step_io_parts(const double *q_in, double *q_out, bool &done, std::string &err);
@@ -155,6 +156,7 @@ struct Solver {
     if (io_graph) { cudaGraphDestroy(io_graph); io_graph = nullptr; }
     io_in = nullptr;
     io_out = nullptr;
+    parts = 0;
   }
   cudaGraph_t io_graph = nullptr;
   cudaGraphExec_t io_graph_exec = nullptr;

@@ -350,10 +350,10 @@ int dg_roe_pair_flux(double gam, int n, const double *qm, const double *qp, cons
  * launches as one chain), 2..32 that many ranges (fewer if the mesh has fewer tiles). */
 void dg_set_step_parts(int parts);
 int dg_step_parts(void);
-/* Steps in one launch of that graph (1..8, default 8; other values select 8), for graphs built from
- * now on: the next step's first face launches of a range then wait only for the element launches
- * whose cells they read (its first element launches for the new dt), so they overlap the previous
- * step's last element launches.  dg_solver_run launches it as often as it fits, then one-step
+/* Steps in one launch of the step graph (1..8, default 8; other values select 8), for graphs built from
+ * now on: with several ranges the next step's first face launches of a range then wait only for the
+ * element launches whose cells they read (its first element launches for the new dt), so they
+ * overlap the previous step's last element launches.  dg_solver_run launches it as often as it fits, then one-step
  * graphs.  Same bits. */
 void dg_set_steps_per_graph(int steps);
 int dg_steps_per_graph(void);
