@@ -35,16 +35,20 @@
 // the dense rows A = [Drw | Dsw | -LIFT/2] (T = 2, parity 0 only: the element kernel's dense form).
 constexpr int kOzRows = 32;  // outputs per parity: up to 4 n-tiles of 8
 constexpr int kOzTables = 3;
+constexpr int kOzSteps = 3, kOzSlots = 16 * kOzSteps;  // k-steps of 16 slots
 __constant__ int c_ozf[kOzTables][7][2][kOzRows];  // biased binary exponent F of every output row: T, order, parity, row
-__device__ uint2 g_ozb[kOzTables][7][2][4][7][2][32];  // B fragments: T, order, parity, n-tile, digit s, k-step, lane
+__device__ uint2 g_ozb[kOzTables][7][2][4][7][kOzSteps][32];  // B fragments: T, order, parity, n-tile, digit s, k-step, lane
 
 // Orders that use the even/odd blocks on the tensor cores: N = 3, 4, 5 (steps on the K=32768
-// O-grid, first form: 365 -> 328, 564 -> 477, 909 -> 720 us).  At N = 1 and 2 the even/odd blocks
+// O-grid, first form: 365 -> 328, 564 -> 477, 909 -> 720 us) and 6 (1142 -> 557 us, with the
+// small tiles; K = 131072 4559 -> 2198 us, K = 256 166 -> 53 us).  At N = 1 and 2 the even/odd blocks
 // were too small a share of the element kernel for the split to pay (N = 1: 184 -> 192 us, N = 2:
-// 236 -> 252 us); those orders use the dense rows instead (ozd_used).  Orders up to 5 fit the
-// exactness bound (at most two k-steps of 16 slots); N = 6 needs three.
-constexpr int kOzMaxN = 5;
-constexpr bool oz_used(int N, bool tc) { return tc && (N == 3 || N == 4 || N == 5); }
+// 236 -> 252 us); those orders use the dense rows instead (ozd_used).  Two k-steps
+// of 16 slots (N <= 5) are within the exactness bound whatever the operator; at N = 6 (39 slots, three
+// k-steps) the operator's own digits keep every level below it, which oz_digits checks.
+constexpr int kOzMaxN = 6;
+// TC: the element kernels' form of elem_tile_sym; at N = 6 every even/odd form contracts there.
+constexpr bool oz_used(int N, int TC) { return N == 6 || (TC != 0 && N >= 3 && N <= 5); }
 // The adjoint element kernel's transposed contraction: N = 3 (the transposed blocks of N = 4
 // need six n-tiles of outputs).
 constexpr bool oz_used_t(int N, bool tc) { return tc && N == 3; }
@@ -60,7 +64,7 @@ constexpr bool ozd_used(int N, int mode) { return mode == 2 && N >= 1 && N <= 2;
 // Minimum resident blocks per SM of an element kernel of form TC (0 FP64, 1 even/odd blocks on the
 // tensor cores, 2 dense rows on the tensor cores) at order N.
 constexpr int elem_min_blocks(int N, int TC) {
-  return (ozd_used(N, TC) || oz_used(N, TC != 0)) ? oz_min_blocks(N) : 1;
+  return (ozd_used(N, TC) || oz_used(N, TC)) ? oz_min_blocks(N) : 1;
 }
 
 __device__ __forceinline__ void mma_f16_16816(float c[4], const uint32_t a[4], const uint2 b) {
@@ -181,7 +185,7 @@ template <int T, int NORD, int K, int R, int SLOT0, int YROW0, int KST, int P, i
           int XST = 128>
 __device__ __forceinline__ void oz_tile(const double *__restrict__ Xd, double *__restrict__ Yd, const int c0,
                                         const int lane, const int *__restrict__ Ems = nullptr) {
-  static_assert(KST <= 2 && K <= 16 * KST && R > 8 * NT && NT < 4, "four n-tiles, two k-steps at most");
+  static_assert(KST <= kOzSteps && K <= 16 * KST && R > 8 * NT && NT < 4, "four n-tiles, three k-steps at most");
   constexpr int SH = PRE ? 2 : 3;  // the alignment shift (oz_align)
   const int g = lane >> 2, t = lane & 3;
   const int col = c0 * 4 + g;  // (cell, variable) of row g; row g + 8 is col + 8
@@ -252,14 +256,14 @@ __device__ __forceinline__ void oz_tile(const double *__restrict__ Xd, double *_
                              oz_pair(hi[0][2], lo[0][2], hi[0][3], lo[0][3], j, v[2]),
                              oz_pair(hi[1][2], lo[1][2], hi[1][3], lo[1][3], j, v[3])};
 #pragma unroll
-      for (int s = 0; s + j < 7; s++) mma_f16_16816(acc[j + s], a, __ldg(bfr + (s * 2 + ks) * 32));
+      for (int s = 0; s + j < 7; s++) mma_f16_16816(acc[j + s], a, __ldg(bfr + (s * kOzSteps + ks) * 32));
     }
   }
   // C fragment: acc[.][0] (row g, col 2t), [1] (g, 2t+1), [2] (g+8, 2t), [3] (g+8, 2t+1).
   // One output: the level sums lev[] of (row g + 8 r, operator row n) joined and rounded.
   auto finish = [&](const float lev[7], const int n, const int r) {
-    // |lev[L]| <= (L + 1) 32 255^2, so that 256 lev[0] + lev[1] and 256 lev[3] + lev[4] (below 2^31 - 6.3e6)
-    // fit 32 bits
+    // |lev[L]| <= (L + 1) 32 255^2 up to N = 5, so that 256 lev[0] + lev[1] and 256 lev[3] + lev[4] (below
+    // 2^31 - 6.3e6) fit 32 bits; at N = 6 by the operator's digits (oz_digits)
     int l[7];
 #pragma unroll
     for (int L = 0; L < 7; L++) l[L] = __float2int_rz(lev[L]);
@@ -481,11 +485,11 @@ static uint32_t oz_f16_bits(int d) {  // |d| <= 255: exact in fp16
 // up to the bits below 2^(F-1023-55) (cut).
 static int oz_digits(const std::vector<double> &S, int NUe, int NUo, int NRe, int NRo, int fexp[2][kOzRows],
                      std::vector<int> &dig, std::string &err) {
-  dig.assign((size_t)2 * 7 * 32 * kOzRows, 0);
+  dig.assign((size_t)2 * 7 * kOzSlots * kOzRows, 0);
   for (int p = 0; p < 2; p++) {
     const int K = p ? NUo : NUe, R = p ? NRo : NRe;
     const size_t base = p ? (size_t)NRe * NUe : 0;
-    if (R > kOzRows || K > 32) { err = "tensor-core contraction: operator too large"; return -4; }
+    if (R > kOzRows || K > kOzSlots) { err = "tensor-core contraction: operator too large"; return -4; }
     for (int n = 0; n < kOzRows; n++) fexp[p][n] = 0;
     for (int n = 0; n < R; n++) {
       int F = 0;
@@ -505,7 +509,18 @@ static int oz_digits(const std::vector<double> &S, int NUe, int NUo, int NRe, in
         const uint64_t m = sh >= 0 ? (M << sh) : (sh > -64 ? (M >> -sh) : 0);
         const int sg = (b >> 63) ? -1 : 1;
         for (int s = 0; s < 7; s++)
-          dig[(((size_t)p * 7 + s) * 32 + k) * kOzRows + n] = sg * (int)((m >> (8 * (6 - s))) & 255);
+          dig[(((size_t)p * 7 + s) * kOzSlots + k) * kOzRows + n] = sg * (int)((m >> (8 * (6 - s))) & 255);
+      }
+      // the largest level sums that any operands (digits up to 255) can give with this row: exact in
+      // FP32 below 2^24, and joined in pairs of 32-bit integers
+      long long lev[7], sum = 0;
+      for (int L = 0; L < 7; L++) {
+        for (int k = 0; k < K; k++) sum += 255ll * std::abs(dig[(((size_t)p * 7 + L) * kOzSlots + k) * kOzRows + n]);
+        lev[L] = sum;
+      }
+      if (lev[6] >= (1ll << 24) || 256 * lev[0] + lev[1] >= (1ll << 31) || 256 * lev[3] + lev[4] >= (1ll << 31)) {
+        err = "tensor-core contraction: level sums beyond the exact range";
+        return -4;
       }
     }
   }
@@ -515,13 +530,13 @@ static int oz_digits(const std::vector<double> &S, int NUe, int NUo, int NRe, in
 // A: the dense rows (Np x NK, row-major) for the dense form's table (T = 2).
 static int oz_upload(int N, const std::vector<double> &S, int NUe, int NUo, int NRe, int NRo,
                      const std::vector<double> &A, int Np, int NK, std::string &err) {
-  if (!oz_used(N, true) && !ozd_used(N, 2)) return 0;
+  if (!oz_used(N, 2) && !ozd_used(N, 2)) return 0;
   static int fexp[kOzTables][2][kOzRows];
-  static uint2 frag[kOzTables][2][4][7][2][32];
+  static uint2 frag[kOzTables][2][4][7][kOzSteps][32];
   std::memset(fexp, 0, sizeof(fexp));
   std::memset(frag, 0, sizeof(frag));
   for (int T = 0; T < kOzTables; T++) {
-    if (T == 0 && !oz_used(N, true)) continue;
+    if (T == 0 && !oz_used(N, 2)) continue;
     if (T == 1 && !oz_used_t(N, true)) continue;
     if (T == 2 && !ozd_used(N, 2)) continue;
     // T = 1: the transposed blocks, S_e^T (NUe x NRe) then S_o^T (NUo x NRo)
@@ -542,10 +557,10 @@ static int oz_upload(int N, const std::vector<double> &S, int NUe, int NUo, int 
     for (int p = 0; p < 2; p++)
       for (int nt = 0; nt < 4; nt++)
         for (int s = 0; s < 7; s++)
-          for (int ks = 0; ks < 2; ks++)
+          for (int ks = 0; ks < kOzSteps; ks++)
             for (int lane = 0; lane < 32; lane++) {
               const int g = lane >> 2, t = lane & 3, k0 = 16 * ks + 2 * t;
-              auto D = [&](int k) { return dig[(((size_t)p * 7 + s) * 32 + k) * kOzRows + 8 * nt + g]; };
+              auto D = [&](int k) { return dig[(((size_t)p * 7 + s) * kOzSlots + k) * kOzRows + 8 * nt + g]; };
               frag[T][p][nt][s][ks][lane].x = oz_f16_bits(D(k0)) | (oz_f16_bits(D(k0 + 1)) << 16);
               frag[T][p][nt][s][ks][lane].y = oz_f16_bits(D(k0 + 8)) | (oz_f16_bits(D(k0 + 9)) << 16);
             }

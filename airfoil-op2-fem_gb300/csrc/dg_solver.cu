@@ -447,9 +447,9 @@ __global__ void __launch_bounds__(32 * np_of(N)) elem_kernel(const Inst d, const
 // differences give y_i - y_P(i).  The contraction shrinks to 0.55-0.62 of the dense one.
 // One tile of 32 cells starting at e0, thread (lane, node i) of a block with at least Np
 // node-warps (warps with i >= Np only take part in the barriers).
-// TC: 0 the even/odd contraction in FP64, 1 the even/odd blocks on the tensor cores (N = 3-5; the
+// TC: 0 the even/odd contraction in FP64 (N = 1-5), 1 the even/odd blocks on the tensor cores (N = 3-6; the
 // butterfly and the operand alignment by oz_prep), 2 the dense rows on the tensor cores at N = 1, 2
-// (no butterfly) and form 1 at N = 3-5.
+// (no butterfly) and the even/odd blocks on the tensor cores at N = 3-6.
 // CT: cells of the tile (32, or 8 or 16 for the tensor-core forms); lane and warp are the thread's
 // place in the block, thread t = 32 warp + lane takes cell t % CT and node t / CT.
 template <int N, bool PDL = false, int TC = 0, int CT = 32>
@@ -460,7 +460,7 @@ __device__ __forceinline__ void elem_tile_sym(const Inst &d, const int stage, co
   constexpr int NPin = NUo;  // input pairs
   constexpr int kS = elem_slot(CT), kS2 = kS / 2;  // doubles and double2 per staged slot
   constexpr bool DENSE = ozd_used(N, TC);           // dense rows, slots in natural order
-  constexpr bool SYMTC = !DENSE && oz_used(N, TC != 0);  // even/odd blocks on the tensor cores
+  constexpr bool SYMTC = !DENSE && oz_used(N, TC);  // even/odd blocks on the tensor cores
   double2 *Y = X + NK * kS2;
   int *Ems = reinterpret_cast<int *>(Y + Np * kS2);  // column exponents of the prepared operands
   static_assert(CT == 32 || DENSE || SYMTC, "small tiles: tensor-core forms only");
@@ -1010,10 +1010,10 @@ static void launch_face(const Inst &d, int stage, cudaStream_t s) {
     launch_pdl(face_kernel<N>, dim3((unsigned)((nf + bs - 1) / bs)), dim3(bs), 0, s, d, stage);
 }
 
-// 3: dense rows on the tensor cores at N = 1, 2 (dg_ozaki.cuh), form 2 at the other orders
-// (default);
-// 2: even/odd with the contraction on the tensor cores (at N = 3, 4, 5, the even/odd FP64
-// kernel at the other orders), 1: even/odd element kernel, 0: dense FP64.
+// 3: dense rows on the tensor cores at N = 1, 2 (dg_ozaki.cuh), the even/odd blocks there at the
+// other orders (default);
+// 2: even/odd with the contraction on the tensor cores (from N = 3 on, in FP64 at N = 1, 2),
+// 1: even/odd in FP64 (on the tensor cores at N = 6), 0: dense FP64.
 static std::atomic<int> g_elem_variant{3};
 
 // The even/odd element kernel instance for form TC at order N, launched over tiles [t0, t1):
@@ -1079,7 +1079,8 @@ static void elem_ws_launch(const Inst &d, int stage, int t0, int t1, cudaStream_
 //   N = 4: 1152 86.2 / 63.8, 8192 114.2 / 112.7, 9600 115.9 / 118.8, 28000 255.7 / 275.9 us
 //   N = 5: 1152 74.9 / 64.6, 3072 88.1 / 96.9, 6000 157.8 / 138.1, 9600 165.9 / 179.2,
 //          28000 423.7 / 410.3, 262144 3784 / 3714 us
-// (N = 5 keeps 32 cells where their blocks, one per SM, nearly fill one or two waves).
+// (N = 5 keeps 32 cells where their blocks, one per SM, nearly fill one or two waves; N = 6, whose
+// 32-cell block would hold 896 threads and 109 KB, has the small tiles only).
 static bool elem_small(int N, int K) {
   switch (N) {
     case 1: return K <= 32768;
@@ -1087,7 +1088,7 @@ static bool elem_small(int N, int K) {
     case 3: return K <= 20480;
     case 4: return K <= 8192;
     case 5: return !((K > 16 * 152 && K <= 32 * 152) || (K > 8192 && K <= 64 * 152));
-    default: return false;
+    default: return true;
   }
 }
 
@@ -1110,7 +1111,7 @@ template <int N>
 static void launch_elem_form(const Inst &d, int stage, int t0, int t1, cudaStream_t s, bool attr) {
   if (t1 <= t0) return;
   if constexpr (elem_small_used(N)) {
-    if (g_elem_variant == 3 && !g_elem_ws && elem_small(N, d.K))
+    if ((g_elem_variant == 3 || N == 6) && !(g_elem_ws && ws_used(N)) && elem_small(N, d.K))
       return elem_small_launch<N>(d, stage, 32 * t0, 32 * t1, s, attr);
   }
   if constexpr (ws_used(N)) {
@@ -1119,7 +1120,7 @@ static void launch_elem_form(const Inst &d, int stage, int t0, int t1, cudaStrea
   if constexpr (ozd_used(N, 2)) {
     if (g_elem_variant == 3) return elem_sym_launch<N, 2, oz_min_blocks(N)>(d, stage, t0, t1, s, attr);
   }
-  if constexpr (oz_used(N, true)) {
+  if constexpr (oz_used(N, 1)) {
     if constexpr (N == 3) {
       // the register budget of two resident blocks per SM instead of three (g_elem_mb)
       if (g_elem_variant >= 2 && g_elem_mb == 2) return elem_sym_launch<N, 1, 2>(d, stage, t0, t1, s, attr);
@@ -1169,7 +1170,7 @@ static cudaError_t set_smem_attr() {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_plain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_sym);
   };
   both(elem_kernel_sym<N, 0, 1, true>, elem_kernel_sym<N, 0, 1, false>);
-  if constexpr (oz_used(N, true))
+  if constexpr (oz_used(N, 1))
     both(elem_kernel_sym<N, 1, oz_min_blocks(N), true>, elem_kernel_sym<N, 1, oz_min_blocks(N), false>);
   if constexpr (N == 3) both(elem_kernel_sym<N, 1, 2, true>, elem_kernel_sym<N, 1, 2, false>);
   if constexpr (ozd_used(N, 2))
@@ -1311,7 +1312,7 @@ static void dense_rows(const Operators &o, std::vector<double> &A) {
 // dimensions, the even/odd operator blocks S, the row exponents and the digits.
 int tc_operator_tables(int N, int dims[4], std::vector<double> &S, int fexp[2][kOzRows], std::vector<int> &dig,
                        std::string &err) {
-  if (!oz_used(N, true)) { err = "no tensor-core contraction at this order"; return -1; }
+  if (!oz_used(N, 1) || N > 5) { err = "no tensor-core tables of 32 slots at this order"; return -1; }
   Operators o;
   if (build_operators(N, o)) { err = "operator construction failed"; return -2; }
   std::vector<double> A;
@@ -1320,7 +1321,12 @@ int tc_operator_tables(int N, int dims[4], std::vector<double> &S, int fexp[2][k
   if (int rc = sym_build(o, A, t, err)) return rc;
   dims[0] = t.NUe; dims[1] = t.NUo; dims[2] = t.NRe; dims[3] = t.NRo;
   S = t.S;
-  return oz_digits(t.S, t.NUe, t.NUo, t.NRe, t.NRo, fexp, dig, err);
+  std::vector<int> all;  // [2][7][kOzSlots][kOzRows], of which the first 32 slots hold all digits
+  if (int rc = oz_digits(t.S, t.NUe, t.NUo, t.NRe, t.NRo, fexp, all, err)) return rc;
+  dig.resize((size_t)2 * 7 * 32 * kOzRows);
+  for (size_t b = 0; b < 2 * 7; b++)
+    std::copy_n(all.begin() + b * kOzSlots * kOzRows, 32 * kOzRows, dig.begin() + b * 32 * kOzRows);
+  return 0;
 }
 
 // Host-only: the tensor-core contraction's final rounding, (th 2^32 + tl) 2^sc to the nearest

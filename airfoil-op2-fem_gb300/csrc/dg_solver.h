@@ -63,8 +63,8 @@ int order_constants_loaded(int dev, int N);
 // 1 if the allocation-free entry point is set up on device dev, 0 if not, -1 out of range.
 int noalloc_ready(int dev);
 // Element kernel form for launches enqueued from now on: 3 (default) tensor cores (dense rows at
-// N = 1, 2, even/odd blocks at N = 3-5), 2 even/odd blocks on the tensor cores at N = 3-5,
-// 1 even/odd FP64, 0 dense FP64.
+// N = 1, 2, even/odd blocks at N = 3-6), 2 even/odd blocks on the tensor cores at N = 3-6,
+// 1 even/odd FP64 (N = 1-5; as 2 at N = 6), 0 dense FP64.
 void set_elem_variant(int v);
 int elem_variant();
 // The tensor-core element form at N = 3 as the warp-specialised persistent kernel: 1 one block

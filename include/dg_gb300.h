@@ -308,9 +308,9 @@ double dg_f16_mma_peak_gflops(void);
 int dg_kernels_per_step(void);
 /* Element-kernel form for launches and graphs built from now on: 3 (default) the dense rows
  * [Drw | Dsw | -LIFT] on the tensor cores as an exact integer product at orders N = 1, 2 and
- * form 2 at the other orders; 2 the even/odd split of those rows with its contraction on the
- * tensor cores at orders N = 3, 4, 5 and in FP64 at the other orders; 1 the even/odd split in
- * FP64; 0 dense FP64 rows.  All compute the same right-hand side to rounding (the tensor-core
+ * the even/odd split there at the other orders; 2 the even/odd split of those rows with its contraction on the
+ * tensor cores from N = 3 on and in FP64 at N = 1, 2; 1 the even/odd split in FP64 (at N = 6 on the
+ * tensor cores, as in forms 2 and 3); 0 dense FP64 rows.  All compute the same right-hand side to rounding (the tensor-core
  * contraction is the correctly rounded dot product of the 56-bit truncated inputs). */
 void dg_set_elem_variant(int variant);
 /* The current element-kernel form. */
