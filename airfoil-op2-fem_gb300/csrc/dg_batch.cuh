@@ -3,8 +3,10 @@
 // operators and the device functions face_node<N> / elem_tile_sym<N> with the plain path: a
 // batched instance computes exactly what its own Solver would, bit for bit.
 //
-// One RK stage of the whole batch is ONE persistent kernel (cooperative launch, all blocks
-// resident):
+// By default one RK stage is a face launch over every instance's face tiles and an element launch per
+// order (grouped launches; small tiles as in the plain path), eight steps per graph launch.  The
+// alternative that the autotuner also times: one RK stage of the whole batch as ONE persistent
+// kernel (cooperative launch, all blocks resident):
 //   phase 1  face tiles of every instance (a tile = up to FT face nodes of one instance)
 //   grid barrier
 //   phase 2  element tiles of every instance (32 cells of one instance; order-4 tiles first)
@@ -117,6 +119,15 @@ __global__ void __launch_bounds__(32 * np_of(N), elem_min_blocks(N, TC)) batch_e
   elem_tile_sym<N, false, TC>(insts[et.x], stage, et.y, threadIdx.x & 31, threadIdx.x >> 5, Xg);
 }
 
+// Grouped element tiles of elem_small_ct(N) cells (see elem_kernel_small).
+template <int N>
+__global__ void __launch_bounds__(elem_small_threads(N), (N <= 3 ? 28 : 24) * 32 / elem_small_threads(N))
+    batch_elem_small_kernel(const Inst *insts, const int4 *etiles, const int first, const int stage) {
+  extern __shared__ double2 Xg[];
+  const int4 et = etiles[first + blockIdx.x];
+  elem_tile_sym<N, false, 2, elem_small_ct(N)>(insts[et.x], stage, et.y, threadIdx.x & 31, threadIdx.x >> 5, Xg);
+}
+
 // The step's finalize of every instance, with the calc_dt maximum taken from the element
 // kernels' single-precision estimates as dt_finalize_kernel does for one solver: fblocks[b] =
 // {instance k, first estimate of the block, blocks of instance k, 0}; each block's 8 warps read
@@ -190,14 +201,26 @@ struct Batch {
   int4 *d_fblocks = nullptr;  // blocks of batch_dt_finalize_kernel
   int nfb = 0;
   int ord_first[7] = {0}, ord_count[7] = {0};  // element tiles of each order (contiguous)
+  bool ord_small[7] = {false};                 // grouped: the order's tiles are small ones
+  long long ord_cells[7] = {0};                // cells of the instances of each order
   GridBarrier *d_bar = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
   cudaGraph_t graph = nullptr;
+  cudaGraphExec_t graphG_exec = nullptr;  // graph_steps steps of grouped launches in one graph
+  cudaGraph_t graphG = nullptr;
+  int graph_steps = 1;
+  int form = -1;  // the element-kernel form that the tiles and graphs were made for
   bool graph_ok = true;
 
+  // Forget the captured step graphs (rebuilt on the next run), e.g. after the shape changed.
+  void drop_graphs() {
+    if (graph_exec) { cudaGraphExecDestroy(graph_exec); graph_exec = nullptr; }
+    if (graph) { cudaGraphDestroy(graph); graph = nullptr; }
+    if (graphG_exec) { cudaGraphExecDestroy(graphG_exec); graphG_exec = nullptr; }
+    if (graphG) { cudaGraphDestroy(graphG); graphG = nullptr; }
+  }
   ~Batch() {
-    if (graph_exec) cudaGraphExecDestroy(graph_exec);
-    if (graph) cudaGraphDestroy(graph);
+    drop_graphs();
     if (d_insts) cudaFree(d_insts);
     if (d_ftiles) cudaFree(d_ftiles);
     if (d_etiles) cudaFree(d_etiles);
@@ -220,6 +243,7 @@ struct Batch {
         return rc;
       }
       maxN = std::max(maxN, cs[k].N);
+      ord_cells[cs[k].N] += s->K;
     }
     maxNp = np_of(maxN);
     std::vector<Inst> insts;
@@ -248,15 +272,20 @@ struct Batch {
     return 0;
   }
 
-  // Element tiles (32 cells of one instance), higher orders first; face tiles of ft nodes.
-  int build_tiles(int ft, std::string &err) {
+  // Element tiles (32 cells of one instance; with grouped launches small tiles where elem_small
+  // chooses them for a mesh of all the order's cells), higher orders first; face tiles of ft nodes.
+  int build_tiles(int ft, bool grouped, std::string &err) {
     std::vector<int4> et, fts;
+    form = g_elem_variant;
     for (int n = 6; n >= 1; n--) {
       ord_first[n] = (int)et.size();
+      ord_small[n] = grouped && (form == 3 || n == 6) &&
+                     elem_small(n, (int)std::min<long long>(ord_cells[n], 0x7FFFFFFF));
+      const int ct = ord_small[n] ? elem_small_ct(n) : 32;
       for (size_t k = 0; k < solvers.size(); k++) {
         if (cfgs[k].N != n) continue;
         const int K = solvers[k]->K;
-        for (int e0 = 0; e0 < K; e0 += 32) et.push_back(make_int4((int)k, e0, 0, n));
+        for (int e0 = 0; e0 < K; e0 += ct) et.push_back(make_int4((int)k, e0, 0, n));
       }
       ord_count[n] = (int)et.size() - ord_first[n];
     }
@@ -304,9 +333,13 @@ struct Batch {
           DG_DISPATCH(n, ce = cudaFuncSetAttribute(batch_elem_kernel<NN, 2>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
         }
+        if (ce == cudaSuccess) {
+          DG_DISPATCH(n, ce = cudaFuncSetAttribute(batch_elem_small_kernel<NN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)elem_sym_smem(NN, elem_small_ct(NN))));
+        }
         if (ce != cudaSuccess) { err = cudaGetErrorString(ce); return -100; }
       }
-      if (int rc = build_tiles(ft, err)) return rc;
+      if (int rc = build_tiles(ft, true, err)) return rc;
       out.variant = variant;
       out.face_tile = ft;
       out.grid = 0;
@@ -325,7 +358,7 @@ struct Batch {
     if (ce == cudaSuccess) ce = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (ce != cudaSuccess) { err = cudaGetErrorString(ce); return -100; }
     if (per_sm < 1) { err = "batched kernel does not fit on an SM"; return -1; }
-    if (int rc = build_tiles(ft, err)) return rc;
+    if (int rc = build_tiles(ft, false, err)) return rc;
     out.variant = variant;
     out.face_tile = ft;
     out.grid = per_sm * sms;
@@ -361,7 +394,11 @@ struct Batch {
     for (int n = 6; n >= 1; n--) {
       if (!ord_count[n]) continue;
       const size_t sm = elem_sym_smem(n);
-      if (g_elem_variant == 3) {
+      if (ord_small[n]) {
+        DG_DISPATCH(n, (batch_elem_small_kernel<NN>
+                        <<<ord_count[n], elem_small_threads(NN), elem_sym_smem(NN, elem_small_ct(NN)), s>>>(
+                            d_insts, d_etiles, ord_first[n], stage)));
+      } else if (g_elem_variant == 3) {
         DG_DISPATCH(n, (batch_elem_kernel<NN, 2><<<ord_count[n], 32 * np_of(NN), sm, s>>>(d_insts, d_etiles,
                                                                                           ord_first[n], stage)));
       } else if (g_elem_variant == 2) {
@@ -441,41 +478,45 @@ struct Batch {
     if (best.variant < 0) { err = "no batched launch shape ran"; return -7; }
     if (int rc = set_shape(best.variant, best.face_tile, shape, err)) return rc;
     shape.ms_per_step = best.ms_per_step;
-    if (graph_exec) { cudaGraphExecDestroy(graph_exec); graph_exec = nullptr; }
-    if (graph) { cudaGraphDestroy(graph); graph = nullptr; }
+    drop_graphs();
     return 0;
   }
 
   int ensure_shape(std::string &err) {
     if (shape.variant >= 0) return 0;
-    const auto vs = batch_variants();
-    for (int v = 0; v < (int)vs.size(); v++)
-      if (vs[v].bs >= 32 * maxNp) return set_shape(v, vs[v].bs, shape, err);
-    err = "no kernel variant fits the batch's highest order";
-    return -1;
+    // Grouped launches with 64-node face tiles: faster than every persistent shape on all sweeps
+    // measured (grouped / the best persistent shape, us per step: 12 O-grids of orders 3 and 4,
+    // 431,884 cells 3198 / 4221; 48 small ones, 57,408 cells 547 / 686; 10 of orders 1-3, 12,012 cells
+    // 116 / 165; of order 2, 151,680 cells 528 / 990; of orders 5 and 6, 151,680 cells 2456 / 3257):
+    // the persistent blocks hold every order's code and idle warps at the lower orders.
+    return set_shape(kGroupedVariant, 64, shape, err);
+  }
+
+  // G steps of grouped launches as one graph.
+  int capture_steps(int G, cudaGraph_t &gr, cudaGraphExec_t &ex, std::string &err) {
+    cudaError_t ce = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
+    if (ce == cudaSuccess)
+      for (int i = 0; i < G; i++) enqueue_step(shape, stream);
+    cudaGraph_t g = nullptr;
+    const cudaError_t ce2 = cudaStreamEndCapture(stream, &g);
+    if (ce == cudaSuccess) ce = ce2;
+    if (ce == cudaSuccess) ce = cudaGraphInstantiate(&ex, g, 0);
+    if (ce != cudaSuccess) {
+      cudaGetLastError();
+      if (g) cudaGraphDestroy(g);
+      ex = nullptr;
+      err = cudaGetErrorString(ce);
+      return -1;
+    }
+    gr = g;
+    return 0;
   }
 
   // The step graph.  Grouped launches are stream-captured; the persistent kernel's graph is
   // built node by node: stream capture does not take cooperative launches, a kernel node with
   // the cooperative attribute does.
   int build_graph(std::string &err) {
-    if (shape.variant == kGroupedVariant) {
-      cudaError_t ce = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
-      if (ce == cudaSuccess) enqueue_step(shape, stream);
-      cudaGraph_t g = nullptr;
-      const cudaError_t ce2 = cudaStreamEndCapture(stream, &g);
-      if (ce == cudaSuccess) ce = ce2;
-      if (ce == cudaSuccess) ce = cudaGraphInstantiate(&graph_exec, g, 0);
-      if (ce != cudaSuccess) {
-        cudaGetLastError();
-        if (g) cudaGraphDestroy(g);
-        graph_exec = nullptr;
-        err = cudaGetErrorString(ce);
-        return -1;
-      }
-      graph = g;
-      return 0;
-    }
+    if (shape.variant == kGroupedVariant) return capture_steps(1, graph, graph_exec, err);
     const BatchVariant v = batch_variants()[shape.variant];
     cudaGraph_t g = nullptr;
     cudaError_t ce = cudaGraphCreate(&g, 0);
@@ -529,11 +570,26 @@ struct Batch {
 
   int run(int nsteps, std::string &err) {
     if (int rc = ensure_shape(err)) return rc;
+    if (!graph_exec && form != g_elem_variant)  // the tiles follow the form until a graph holds them
+      if (int rc = set_shape(shape.variant, shape.face_tile, shape, err)) return rc;
     if (!graph_exec && graph_ok) {
       std::string gerr;
       if (build_graph(gerr)) graph_ok = false;  // launch directly instead
     }
-    for (int i = 0; i < nsteps; i++) {
+    int i = 0;
+    if (graph_exec && shape.variant == kGroupedVariant) {
+      // several steps per graph launch, as the plain solver (see g_steps_per_graph)
+      std::string gerr;
+      if (!graphG_exec) graph_steps = steps_per_graph();
+      if (graph_steps > 1 && nsteps >= graph_steps && !graphG_exec && form == g_elem_variant)
+        capture_steps(graph_steps, graphG, graphG_exec, gerr);
+      if (graphG_exec)
+        for (; i + graph_steps <= nsteps; i += graph_steps) {
+          cudaError_t ce = cudaGraphLaunch(graphG_exec, stream);
+          if (ce != cudaSuccess) { err = std::string("batched step: ") + cudaGetErrorString(ce); return -100; }
+        }
+    }
+    for (; i < nsteps; i++) {
       cudaError_t ce = graph_exec ? cudaGraphLaunch(graph_exec, stream) : enqueue_step(shape, stream);
       if (ce != cudaSuccess) { err = std::string("batched step: ") + cudaGetErrorString(ce); return -100; }
     }

@@ -2354,8 +2354,7 @@ extern "C" int dg_batch_use_shape(dg_batch_t *h, int variant, int face_tile) {
   dg::BatchShape sh;
   if (h->b.set_shape(variant, face_tile, sh, err)) return batch_fail(DG_ERR_ARG, err);
   h->b.shape = sh;
-  if (h->b.graph_exec) { cudaGraphExecDestroy(h->b.graph_exec); h->b.graph_exec = nullptr; }
-  if (h->b.graph) { cudaGraphDestroy(h->b.graph); h->b.graph = nullptr; }
+  h->b.drop_graphs();
   h->b.graph_ok = true;
   return 0;
 }

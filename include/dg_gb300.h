@@ -156,9 +156,10 @@ void dg_solver_free(dg_solver_t *s);
 
 /* ------------------------------------------------------------------ batched instances
  * Many instances (airfoil or vortex, any size, order 1..6, Mach, alpha) advanced together:
- * each RK stage of the whole batch is one persistent kernel (cooperative launch: face phase,
- * grid barrier, element phase over all instances' tiles), a step is three of them plus one
- * finalize, captured in a CUDA graph.  Each instance computes exactly what dg_solver would.
+ * each RK stage of the whole batch is one face launch over all instances' face tiles and one element
+ * launch per order (grouped launches, the default), or one persistent kernel (cooperative launch:
+ * face phase, grid barrier, element phase over all instances' tiles); a step is three stages plus
+ * one finalize, captured in a CUDA graph.  Each instance computes exactly what dg_solver would.
  * A grid barrier wait is bounded (about 2 s); if one gives up, dg_batch_sync reports it. */
 typedef struct dg_batch_t dg_batch_t;
 int dg_batch_create(int n, const dg_config_t *cfgs, const dg_mesh_t *const *meshes, dg_batch_t **out);
