@@ -2,14 +2,15 @@
 // dg_solver.cu: it shares the per-order operators [Drw | Dsw | -LIFT/2] in constant memory, the
 // reference-node coordinates, the affine geometry kernel and the edge records of the Euler path.
 //
-// One classical RK4 stage is two kernels:
+// One classical RK4 stage is one kernel, advec_fused_kernel (below).  The forms that element-kernel
+// forms 0 and (at N = 3) 1 select have two:
 //   advec_face_kernel  one thread per face node (boundary faces first): the Lax-Friedrichs flux
 //                      n.(F- + F+)/2 + |v|(q- - q+)/2 of advec/src/advec_rhs.h:36-63 once per
 //                      face node, with the trace of the neighbour (advec/src/get_neighbour_q.h)
 //                      or the constant ghost value 4.5e-5 (advec/src/get_bedge_q.h), written
 //                      into both cells' face slots scaled by each side's fscale (twice the flux:
 //                      the 1/2 is in the operator's LIFT columns);
-//   advec_elem_kernel  32 cells x Np node-warps (even/odd form by default, advec_elem_kernel_sym):
+//   advec_elem_kernel  32 cells x Np node-warps (even/odd form advec_elem_kernel_sym):
 //                      rhs = cr Drw q + cs Dsw q - LIFT flux with
 //                      cr = vx rx + vy ry, cs = vx sx + vy sy (F = vx q, G = vy q on affine
 //                      cells; advec_rhs.h:11-34), then the RK4 combine: W = q + dt frac k for
@@ -18,6 +19,8 @@
 //                      k1 + 2 k2 + 2 k3 is accumulated in one array in the reference's order.
 // Layout: q, W, acc [K][Np]; flux [K][3][Nfp].  dt is fixed; t is kept on the host.
 #pragma once
+
+#include <type_traits>
 
 #include "dg_advec.h"
 
@@ -201,81 +204,120 @@ __global__ void __launch_bounds__(32 * np_of(N)) advec_elem_kernel_sym(const Adv
   }
 }
 
-// The element kernel with the even/odd contraction on the tensor cores (the exact integer
-// product of dg_ozaki.cuh): one variable per column, so a 32-cell tile is two row tiles of 16
-// cells and the units are (row tile, n-tile of outputs).  Staging, butterfly and alignment
-// (oz_prep over 64 threads), the contraction, the recombination and the RK4 combine follow
-// advec_elem_kernel_sym; the right-hand side equals it to rounding.  Used at N = 3 (K = 524288:
-// 0.304 -> 0.254 ms per stage, step 1.45 -> 1.20 ms); at N = 4, 5 a tile has only 6 or 8
-// contraction units for 15 or 21 warps and measured slower than the FP64 kernel (0.562 vs 0.537,
-// 0.931 vs 0.885 ms per stage), so those orders keep it.
-constexpr bool advec_tc(int N) { return N == 3; }
+// One RK4 stage in one kernel, the contraction on the tensor cores (the exact integer product of
+// dg_ozaki.cuh; dense rows at N = 1, 2, the even/odd blocks from N = 3 on).  A block takes NC cells, one
+// column each (16 columns per row tile):
+//   1. stages [cr W; cs W] and the face terms.  The velocity is constant, so a side's scaled flux is
+//      A q- + B q+ with A = fscale (v.n + |v|), B = fscale (v.n - |v|) per cell face (AdvInst::coef): two
+//      FP64 instructions on the trace values, read from W in place.  Each side forms its own flux;
+//      a face kernel's flux array (a write and a read of 3 Nfp values per cell and stage) and its
+//      launch are not needed, at the price of reading W of one buffer and writing another.
+//   2. operand pre-pass, contraction, 3. recombination and the RK4 combine of advec_elem_kernel.
+// ~120 FP64 instructions per cell at N = 4 (100 us of the 260 us stage at K = 524288); the rest is the
+// integer work of the exact product.  Step at K = 524288, N = 1 / 2 / 3 / 4: 404 / 800 / 1083 / 2449 ->
+// 283 / 461 / 716 / 1039 us; K = 259200, N = 5 / 6: 1960 / 3093 -> 952 / 1231 us (before: a face kernel and
+// an element kernel in FP64, on the tensor cores at N = 3).
 template <int N>
-__global__ void __launch_bounds__(32 * np_of(N), oz_min_blocks(N)) advec_elem_kernel_tc(const AdvInst d,
-                                                                                         const int stage) {
-  constexpr int Np = np_of(N), NF = 3 * (N + 1), NK = nk_of(N);
+constexpr size_t advec_fused_smem(int NC) {
+  return (size_t)(nk_of(N) + np_of(N)) * (NC + 2) * sizeof(double) + NC * sizeof(int);
+}
+constexpr int advec_fused_threads(int NC) { return NC == 16 ? 128 : 256; }
+
+template <int N, int NC>
+__global__ void __launch_bounds__(advec_fused_threads(NC), 768 / advec_fused_threads(NC))
+    advec_fused_kernel(const AdvInst d, const int stage, const double *__restrict__ in, double *__restrict__ out) {
+  constexpr int Np = np_of(N), Nfp = N + 1, NF = 3 * Nfp, NK = nk_of(N), XS = NC + 2;
   constexpr int NUe = Sym<N>::NUe, NUo = Sym<N>::NUo, NRe = Sym<N>::NRe, NRo = Sym<N>::NRo;
-  // 32 cells + 4 doubles of padding per slot: the fragment loads' four k-rows fall on different banks
-  constexpr int XS = 36;
-  constexpr int NTT = (NRe + 7) / 8 + (NRo + 7) / 8;  // n-tiles of outputs
-  __shared__ __align__(16) double X[NK * XS];  // [slot][cell]
-  __shared__ __align__(16) double Y[Np * XS];  // even / odd row results [row][cell]
-  __shared__ double R[32 * Np];                // right-hand sides [cell][node]
-  __shared__ int Ems[32];                      // column exponents of the prepared operands
-  const int t = threadIdx.x;
-  const int e0 = blockIdx.x * 32;
-  const int nc = min(32, d.K - e0);
+  constexpr bool DENSE = N <= 2;
+  constexpr int T = advec_fused_threads(NC);
+  extern __shared__ __align__(16) double Xf[];  // [NK][XS]: slot, cell
+  double *Y = Xf + NK * XS;                      // [Np][XS]: rows, cell
+  int *Ems = reinterpret_cast<int *>(Y + Np * XS);
+  __shared__ int s_pos[NK], s_fm[NF], s_out[Np];  // staging slots, face nodes, recombination
+  const int t = threadIdx.x, e0 = blockIdx.x * NC, nc = min(NC, d.K - e0);
+  for (int k = t; k < NK; k += T) s_pos[k] = (DENSE ? k : c_pos[N][k]) * XS;
+  for (int k = t; k < NF; k += T) s_fm[k] = d.fmask[k];
+  for (int k = t; k < Np; k += T)  // even row, odd row + 1 (0: none), sign
+    s_out[k] = c_out[N][3 * k] | ((c_out[N][3 * k + 1] + 1) << 8) | (c_out[N][3 * k + 2] > 0 ? 1 << 16 : 0);
+  __syncthreads();
   const size_t base = (size_t)e0 * Np;
-  {
-    const int el = t / Np, k = t - el * Np;
-    double cr = 0.0, cs = 0.0, w = 0.0;
+  for (int j = t; j < NC * Np; j += T) {
+    const int el = j / Np, k = j - el * Np;
+    double2 c = make_double2(0.0, 0.0);
+    double w = 0.0;
     if (el < nc) {
-      const double *g = d.geo + (size_t)(e0 + el) * 16;
-      cr = d.vx * g[0] + d.vy * g[1];
-      cs = d.vx * g[2] + d.vy * g[3];
-      w = d.W[base + t];
+      c = ld2(d.coef + (size_t)(e0 + el) * 8);
+      w = in[base + j];
     }
-    X[c_pos[N][k] * XS + el] = cr * w;
-    X[c_pos[N][Np + k] * XS + el] = cs * w;
-    for (int j = t; j < 32 * NF; j += 32 * Np) {
-      const int ef = j / NF, f = j - ef * NF;
-      X[c_pos[N][2 * Np + f] * XS + ef] = ef < nc ? d.flux[(size_t)e0 * NF + j] : 0.0;
+    Xf[s_pos[k] + el] = c.x * w;
+    Xf[s_pos[Np + k] + el] = c.y * w;
+  }
+  for (int j = t; j < NC * NF; j += T) {
+    const int el = j / NF, f = j - el * NF, fc = f / Nfp, i = f - fc * Nfp;
+    double v = 0.0;
+    if (el < nc) {
+      const size_t e = e0 + el;
+      const int2 nb = __ldg(&d.nbr[3 * e + fc]);  // {cell or -1, face | reverse << 2}
+      const double2 c = ld2(d.coef + e * 8 + 2 + 2 * fc);
+      const double qm = in[e * Np + s_fm[f]];
+      const int ir = (nb.y >> 2) ? Nfp - 1 - i : i;
+      const double qp = nb.x < 0 ? kAdvecGhost : in[(size_t)nb.x * Np + s_fm[(nb.y & 3) * Nfp + ir]];
+      v = fma(c.x, qm, c.y * qp);
     }
+    Xf[s_pos[2 * Np + f] + el] = v;
   }
   __syncthreads();
-  oz_prep<NUe, NUo, XS, 32>(X, Ems, t);
-  __syncthreads();
-  const int lane = t & 31, i = t >> 5;
-  // unit u: n-tile u >> 1 of the outputs (even rows first), cells 16 (u & 1) .. + 15
-  for (int u = i; u < 2 * NTT; u += Np)
-    oz_unit<N, 0, NUe, NRe, NUo, NRo, NUe, NRe, 0, true, XS>(X, Y, u >> 1, (u & 1) * 4, lane, Ems);
-  __syncthreads();
-  {
-    const int re = c_out[N][3 * i], ro = c_out[N][3 * i + 1], sg = c_out[N][3 * i + 2];
-    double r = Y[re * XS + lane];
-    if (ro >= 0) r = sg > 0 ? r + Y[ro * XS + lane] : r - Y[ro * XS + lane];
-    R[lane * Np + i] = r;
-  }
-  __syncthreads();
-  const int el = t / Np;
-  if (el >= nc) return;
-  const size_t o = base + t;
-  const double r = R[t];
-  if (stage == 4) {
-    d.rhs_out[o] = r;
-    return;
-  }
-  const double q = d.q[o], dt = d.dt;
-  if (stage == 0) {
-    d.acc[o] = r;
-    d.W[o] = __dadd_rn(q, __dmul_rn(dt * 0.5, r));
-  } else if (stage < 3) {
-    d.acc[o] = __dadd_rn(d.acc[o], 2.0 * r);
-    d.W[o] = __dadd_rn(q, __dmul_rn(stage == 1 ? dt * 0.5 : dt, r));
+  const int lane = t & 31, warp = t >> 5;
+  if constexpr (DENSE) {
+    oz_product<N, 2, NK, Np, 0, 0, NK, Np, false, XS, NC / 16>(Xf, Y, warp, T / 32, lane);
   } else {
-    const double qn = __dadd_rn(q, __dmul_rn((1.0 / 6.0) * dt, __dadd_rn(d.acc[o], r)));
-    d.q[o] = qn;
-    d.W[o] = qn;
+    oz_prep<NUe, NUo, XS, NC, T / NC>(Xf, Ems, t);
+    __syncthreads();
+    oz_product<N, 0, NUe, NRe, NUo, NRo, NUe, NRe, true, XS, NC / 16>(Xf, Y, warp, T / 32, lane, Ems);
+  }
+  __syncthreads();
+  for (int j = t; j < nc * Np; j += T) {
+    const int el = j / Np, i = j - el * Np;
+    double r;
+    if constexpr (DENSE) {
+      r = Y[i * XS + el];
+    } else {
+      const int o = s_out[i], ro = ((o >> 8) & 0xFF) - 1;
+      r = Y[(o & 0xFF) * XS + el];
+      if (ro >= 0) r = (o >> 16) ? r + Y[ro * XS + el] : r - Y[ro * XS + el];
+    }
+    const size_t o = base + j;
+    if (stage == 4) {
+      d.rhs_out[o] = r;
+      continue;
+    }
+    const double q = d.q[o], dt = d.dt;
+    if (stage == 0) {
+      d.acc[o] = r;
+      out[o] = __dadd_rn(q, __dmul_rn(dt * 0.5, r));
+    } else if (stage < 3) {
+      d.acc[o] = __dadd_rn(d.acc[o], 2.0 * r);
+      out[o] = __dadd_rn(q, __dmul_rn(stage == 1 ? dt * 0.5 : dt, r));
+    } else {
+      const double qn = __dadd_rn(q, __dmul_rn((1.0 / 6.0) * dt, __dadd_rn(d.acc[o], r)));
+      d.q[o] = qn;
+      out[o] = qn;
+    }
+  }
+}
+
+// The coefficients of AdvInst::coef for each cell: cr, cs, then (A, B) of faces 0..2.
+__global__ void advec_coef_kernel(const AdvInst d, double *coef) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= d.K) return;
+  const double *g = d.geo + (size_t)e * 16;
+  double *c = coef + (size_t)e * 8;
+  c[0] = d.vx * g[0] + d.vy * g[1];
+  c[1] = d.vx * g[2] + d.vy * g[3];
+  for (int f = 0; f < 3; f++) {
+    const double vn = d.vx * g[4 + 3 * f] + d.vy * g[5 + 3 * f], fs = g[6 + 3 * f];
+    c[2 + 2 * f] = fs * (vn + d.speed);
+    c[3 + 2 * f] = fs * (vn - d.speed);
   }
 }
 
@@ -309,30 +351,59 @@ __global__ void advec_vertex_kernel(int K, const int *cells, const int *owner, c
   }
 }
 
-// Element-kernel forms 2 and 3 use the tensor-core contraction where advec_tc says, form 1 (and
-// forms 2, 3 at the other orders) the even/odd FP64 kernel, form 0 the dense FP64 kernel.
+// Element-kernel forms 2 and 3, and at every order but 3 form 1, run advec_fused_kernel; form 1 at
+// N = 3 the face kernel and the even/odd FP64 kernel, form 0 the face kernel and the dense one.
+static bool advec_fused(int N) { return g_elem_variant >= (N == 3 ? 2 : 1); }
+
 template <int N>
 static void advec_launch_elem(const AdvInst &d, int stage, cudaStream_t s) {
-  if constexpr (advec_tc(N)) {
-    if (g_elem_variant >= 2) {
-      advec_elem_kernel_tc<N><<<(d.K + 31) / 32, 32 * np_of(N), 0, s>>>(d, stage);
+  if constexpr (N == 3) {
+    if (g_elem_variant) {
+      advec_elem_kernel_sym<N><<<(d.K + 31) / 32, 32 * np_of(N), 0, s>>>(d, stage);
       return;
     }
   }
-  if (g_elem_variant) advec_elem_kernel_sym<N><<<(d.K + 31) / 32, 32 * np_of(N), 0, s>>>(d, stage);
-  else advec_elem_kernel<N><<<(d.K + 31) / 32, 32 * np_of(N), 0, s>>>(d, stage);
+  advec_elem_kernel<N><<<(d.K + 31) / 32, 32 * np_of(N), 0, s>>>(d, stage);
+}
+
+// Stages 0..2 write the buffer that they do not read (W and W2 in turn), so that W holds the state
+// after a step as before; the right-hand side alone (4) writes neither.
+template <int N>
+static void advec_launch_fused(const AdvInst &d, int stage, cudaStream_t s) {
+  const double *in = (stage == 1 || stage == 3) ? d.W2 : d.W;
+  double *out = (stage == 0 || stage == 2) ? d.W2 : d.W;
+  auto go = [&](auto nc) {
+    constexpr int NC = decltype(nc)::value;
+    advec_fused_kernel<N, NC><<<(d.K + NC - 1) / NC, advec_fused_threads(NC), advec_fused_smem<N>(NC), s>>>(d, stage, in, out);
+  };
+  // Few cells: blocks of 16 (one row tile) spread them over the SMs.  Step, 16 / 128 cells a block:
+  // K = 1152 24.8 / 47.1 us (N = 3), 29.9 / 69.4 (N = 4); K = 8192 29.6 / 49.0, 39.9 / 71.4; K = 16200
+  // 55.4 / 49.7, 70.3 / 72.4; K = 32768 79.8 / 63.3, 107.3 / 91.4 us.
+  if (d.K <= 12288) go(std::integral_constant<int, 16>());
+  else go(std::integral_constant<int, 128>());
+}
+
+template <int N>
+static void advec_launch_face(const AdvInst &d, cudaStream_t s) {
+  const int nf = (d.nE + d.nB) * (N + 1);
+  if (nf) advec_face_kernel<N><<<(nf + 255) / 256, 256, 0, s>>>(d);
 }
 
 template <int N>
 static void advec_launch_stage(const AdvInst &d, int stage, cudaStream_t s) {
-  const int nf = (d.nE + d.nB) * (N + 1);
-  if (nf) advec_face_kernel<N><<<(nf + 255) / 256, 256, 0, s>>>(d);
-  advec_launch_elem<N>(d, stage, s);
+  if (advec_fused(N)) {
+    advec_launch_fused<N>(d, stage, s);
+  } else {
+    advec_launch_face<N>(d, s);
+    advec_launch_elem<N>(d, stage, s);
+  }
 }
 
 Advection::~Advection() {
   if (graph_exec) cudaGraphExecDestroy(graph_exec);
   if (graph) cudaGraphDestroy(graph);
+  if (graphG_exec) cudaGraphExecDestroy(graphG_exec);
+  if (graphG) cudaGraphDestroy(graphG);
   for (void *p : allocs) cudaFree(p);
   if (stream) cudaStreamDestroy(stream);
 }
@@ -370,10 +441,21 @@ int Advection::create(const Mesh &m, int order, double vel_x, double vel_y, doub
   const size_t nq = (size_t)K * Np;
   d.q = (double *)alloc(nq * 8);
   d.W = (double *)alloc(nq * 8);
+  d.W2 = (double *)alloc(nq * 8);
   d.acc = (double *)alloc(nq * 8);
   d.flux = (double *)alloc((size_t)K * 3 * Nfp * 8);
   double *geo = (double *)alloc((size_t)K * 16 * 8);
   d.geo = geo;
+  double *coef = (double *)alloc((size_t)K * 8 * 8);
+  d.coef = coef;
+  int2 *nbr = (int2 *)alloc((size_t)K * 3 * sizeof(int2));
+  d.nbr = nbr;
+  std::vector<int2> nb((size_t)K * 3, make_int2(-1, 0));
+  for (const int4 &e : edges) {
+    const int fL = e.z & 3, fR = (e.z >> 2) & 3, rev = (e.z >> 4) & 1;
+    nb[3 * (size_t)e.x + fL] = make_int2(e.y, fR | (rev << 2));
+    nb[3 * (size_t)e.y + fR] = make_int2(e.x, fL | (rev << 2));
+  }
   int4 *de = (int4 *)alloc(sizeof(int4) * d.nE), *db = (int4 *)alloc(sizeof(int4) * d.nB);
   d.edges = de;
   d.bedges = db;
@@ -381,7 +463,8 @@ int Advection::create(const Mesh &m, int order, double vel_x, double vel_y, doub
   d.fmask = fm;
   coords_d = (double *)alloc(m.coords.size() * 8);
   cells_d = (int *)alloc(m.cell2nodes.size() * 4);
-  for (void *p : {(void *)d.q, (void *)d.W, (void *)d.acc, (void *)d.flux, (void *)geo, (void *)de, (void *)db,
+  for (void *p : {(void *)d.q, (void *)d.W, (void *)d.W2, (void *)d.acc, (void *)d.flux, (void *)geo, (void *)coef,
+                  (void *)nbr, (void *)de, (void *)db,
                   (void *)fm, (void *)coords_d, (void *)cells_d})
     if (!p) { err = "cudaMalloc failed"; return -101; }
   CK(cudaMemcpyAsync(de, edges.data(), sizeof(int4) * d.nE, cudaMemcpyHostToDevice, stream));
@@ -391,8 +474,12 @@ int Advection::create(const Mesh &m, int order, double vel_x, double vel_y, doub
   CK(cudaMemcpyAsync(cells_d, m.cell2nodes.data(), m.cell2nodes.size() * 4, cudaMemcpyHostToDevice, stream));
   CK(cudaMemsetAsync(d.flux, 0, (size_t)K * 3 * Nfp * 8, stream));
   CK(cudaMemsetAsync(d.acc, 0, nq * 8, stream));
+  CK(cudaMemcpyAsync(nbr, nb.data(), nb.size() * sizeof(int2), cudaMemcpyHostToDevice, stream));
   geometry_kernel<<<(K + 127) / 128, 128, 0, stream>>>(K, coords_d, cells_d, geo);
+  advec_coef_kernel<<<(K + 127) / 128, 128, 0, stream>>>(d, coef);
   CK(cudaGetLastError());
+  DG_DISPATCH(N, CK(cudaFuncSetAttribute(advec_fused_kernel<NN, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)advec_fused_smem<NN>(128))));  // 16 cells need 16 KB at most
   CK(cudaStreamSynchronize(stream));
   return 0;
 }
@@ -412,30 +499,42 @@ void Advection::enqueue_step(cudaStream_t s) {
 }
 
 void Advection::enqueue_step_events(cudaStream_t s, cudaEvent_t *ev) {
-  const int nf = (d.nE + d.nB) * (N + 1);
   for (int stage = 0; stage < 4; stage++) {
-    DG_DISPATCH(N, (advec_face_kernel<NN><<<(nf + 255) / 256, 256, 0, s>>>(d)));
+    if (!advec_fused(N)) DG_DISPATCH(N, advec_launch_face<NN>(d, s));
     cudaEventRecord(ev[1 + 2 * stage], s);
-    DG_DISPATCH(N, advec_launch_elem<NN>(d, stage, s));
+    if (advec_fused(N)) {
+      DG_DISPATCH(N, advec_launch_fused<NN>(d, stage, s));
+    } else {
+      DG_DISPATCH(N, advec_launch_elem<NN>(d, stage, s));
+    }
     cudaEventRecord(ev[2 + 2 * stage], s);
   }
 }
 
 int Advection::step(int nsteps, bool use_graph, std::string &err) {
-  if (use_graph && !graph_exec) {
+  auto capture = [&](int G, cudaGraph_t &g, cudaGraphExec_t &ex) -> int {
+    if (ex) return 0;
     CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    enqueue_step(stream);
-    cudaError_t ce = cudaStreamEndCapture(stream, &graph);
+    for (int k = 0; k < G; k++) enqueue_step(stream);
+    cudaError_t ce = cudaStreamEndCapture(stream, &g);
     if (ce != cudaSuccess) { err = std::string("graph capture: ") + cudaGetErrorString(ce); return -6; }
-    CK(cudaGraphInstantiate(&graph_exec, graph, 0));
+    CK(cudaGraphInstantiate(&ex, g, 0));
+    return 0;
+  };
+  int i = 0;
+  if (use_graph && nsteps >= kGraphSteps) {
+    if (int rc = capture(kGraphSteps, graphG, graphG_exec)) return rc;
+    for (; i + kGraphSteps <= nsteps; i += kGraphSteps) CK(cudaGraphLaunch(graphG_exec, stream));
   }
-  for (int i = 0; i < nsteps; i++) {
+  if (use_graph && i < nsteps)
+    if (int rc = capture(1, graph, graph_exec)) return rc;
+  for (; i < nsteps; i++) {
     if (use_graph) CK(cudaGraphLaunch(graph_exec, stream));
     else enqueue_step(stream);
-    t += d.dt;  // advec/src/advec.cpp:262
-    steps++;
   }
   CK(cudaGetLastError());
+  for (int k = 0; k < nsteps; k++) t += d.dt;  // advec/src/advec.cpp:262
+  steps += (unsigned long long)nsteps;
   return 0;
 }
 

@@ -16,7 +16,9 @@ struct AdvInst {
   const int4 *bedges;  // {cell, face, type, 0}
   const int *fmask;
   const double *geo;   // [K][16]: rx, ry, sx, sy, (nx, ny, fscale) x 3, J, pad
-  double *q, *W, *acc, *flux, *rhs_out;
+  const double *coef;  // [K][8]: cr, cs, then A, B of each face (advec_fused_kernel)
+  const int2 *nbr;     // [K][3]: {neighbour cell or -1, its face | reverse << 2}
+  double *q, *W, *W2, *acc, *flux, *rhs_out;
   double vx, vy, speed, dt;
 };
 
@@ -28,6 +30,9 @@ struct Advection {
   cudaStream_t stream = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
+  static constexpr int kGraphSteps = 8;  // steps of the longer graph that runs launch where it fits
+  cudaGraph_t graphG = nullptr;
+  cudaGraphExec_t graphG_exec = nullptr;
   double *coords_d = nullptr;
   int *cells_d = nullptr;
   std::vector<void *> allocs;
@@ -36,7 +41,8 @@ struct Advection {
   int create(const Mesh &m, int order, double vel_x, double vel_y, double dt, std::string &err);
   int init(std::string &err);
   void enqueue_step(cudaStream_t s);
-  // One step with an event after each of its eight kernels (ev[0] recorded by the caller).
+  // One step with two events per stage, after its face launch (none with the fused kernel) and at its
+  // end (ev[0] recorded by the caller).
   void enqueue_step_events(cudaStream_t s, cudaEvent_t *ev);
   int step(int nsteps, bool use_graph, std::string &err);
   int rhs(double *out_dev, std::string &err);

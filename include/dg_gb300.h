@@ -141,7 +141,8 @@ int dg_advec_set(dg_advec_t *a, const char *name, const double *host);  /* q, wo
 /* One right-hand side of W (advec_rhs after the face loops); overwrites workingQ. */
 int dg_advec_rhs(dg_advec_t *a, const double *W, double *rhs);
 int dg_advec_time(dg_advec_t *a, double *t, unsigned long long *steps);
-/* One step as separate launches with per-kernel times (face, element) x 4 stages, in ms. */
+/* One step as separate launches with per-kernel times (face, element) x 4 stages, in ms; with the fused
+ * stage kernel (the default) the face entries are empty intervals and the element entries the stage. */
 int dg_advec_step_timed(dg_advec_t *a, float *ms8);
 /* q per mesh vertex as advec/src/save_solution.cpp:13-52 samples it, and as a legacy-VTK file. */
 int dg_advec_vertex_values(dg_advec_t *a, const dg_mesh_t *mesh, double *out);
