@@ -332,31 +332,21 @@ __device__ __forceinline__ void nodal_flux_adj(const double gm1, const double w0
                                                const double w3, const double rx, const double ry, const double sx,
                                                const double sy, const double2 r01, const double2 r23,
                                                const double2 s01, const double2 s23, double *out) {
-  const double ir = rcp(w0);
+  // ~50 FP64 instructions (each sum a chain of fused multiply-adds)
+  const double ir = rcp_seeded(w0);
   const double u = w1 * ir, v = w2 * ir;
-  const double p = gm1 * fma(-0.5, fma(w1, u, w2 * v), w3);
-  const double ep = w3 + p;
+  const double ep = fma(gm1, fma(-0.5, fma(w1, u, w2 * v), w3), w3);
   const double U = fma(rx, u, ry * v), V = fma(sx, u, sy * v);
-  double w1b = rx * r01.x + sx * s01.x, w2b = ry * r01.x + sy * s01.x;
-  w1b += r01.y * U + s01.y * V;
-  w2b += r23.x * U + s23.x * V;
-  const double Ub = r01.y * w1 + r23.x * w2 + r23.y * ep;
-  const double Vb = s01.y * w1 + s23.x * w2 + s23.y * ep;
-  double pb = rx * r01.y + ry * r23.x + sx * s01.y + sy * s23.x;
-  const double epb = r23.y * U + s23.y * V;
-  double w3b = epb;
-  pb += epb;
-  double ub = rx * Ub + sx * Vb, vb = ry * Ub + sy * Vb;
-  w3b += gm1 * pb;
-  const double kk = -0.5 * gm1 * pb;
-  w1b += kk * u;
-  ub += kk * w1;
-  w2b += kk * v;
-  vb += kk * w2;
-  w1b += ub * ir;
-  w2b += vb * ir;
-  const double irb = ub * w1 + vb * w2;
-  const double w0b = -irb * ir * ir;
+  const double Ub = fma(r23.y, ep, fma(r23.x, w2, r01.y * w1));
+  const double Vb = fma(s23.y, ep, fma(s23.x, w2, s01.y * w1));
+  const double epb = fma(s23.y, V, r23.y * U);
+  const double pb = fma(sy, s23.x, fma(sx, s01.y, fma(ry, r23.x, fma(rx, r01.y, epb))));
+  const double w3b = fma(gm1, pb, epb);
+  const double kk = (-0.5 * gm1) * pb;
+  const double ub = fma(kk, w1, fma(sx, Vb, rx * Ub)), vb = fma(kk, w2, fma(sy, Vb, ry * Ub));
+  const double w1b = fma(ub, ir, fma(kk, u, fma(s01.y, V, fma(r01.y, U, fma(sx, s01.x, rx * r01.x)))));
+  const double w2b = fma(vb, ir, fma(kk, v, fma(s23.x, V, fma(r23.x, U, fma(sy, s01.x, ry * r01.x)))));
+  const double w0b = -fma(ub, u, vb * v) * ir;
   st2(out, w0b, w1b);
   st2(out + 2, w2b, w3b);
 }

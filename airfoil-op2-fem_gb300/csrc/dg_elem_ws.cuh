@@ -139,7 +139,7 @@ __device__ __forceinline__ void ws_compute(const Inst &d, const int e0, const in
   const double rx = gv[0].x, ry = gv[0].y, sx = gv[1].x, sy = gv[1].y;
   double fr0 = 0, fr1 = 0, fr2 = 0, fr3 = 0, fs0 = 0, fs1 = 0, fs2 = 0, fs3 = 0;
   if (live) {
-    const double ir = rcp(w[0]);
+    const double ir = rcp_seeded(w[0]);
     const double u = w[1] * ir, v = w[2] * ir;
     const double p = P.gm1 * fma(-0.5, fma(w[1], u, w[2] * v), w[3]);
     const double ep = w[3] + p;

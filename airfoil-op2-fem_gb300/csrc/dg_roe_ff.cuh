@@ -195,6 +195,23 @@ DG_HD double dbl_from(const float v) {
   return bits_dbl(a < 0x00800000u ? 0ull : r);
 }
 
+// 1 / x within a rounding or two of the nearest double, from a float seed: y (1 + e + e^2), e = 1 - x y
+// (e < 2^-21, the cut term below 2^-63).  Three FP64 instructions; __drcp_rn takes five and is used
+// outside 2^-100 .. 2^100 (zero, non-finite values among the rest).
+DG_HD double rcp_seeded(const double x) {
+  const uint32_t a = (uint32_t)(dbl_bits(x) >> 32) & 0x7FFFFFFFu;
+  if (a - ((1023u - 100u) << 20) >= (200u << 20)) {
+#ifdef __CUDA_ARCH__
+    return __drcp_rn(x);
+#else
+    return 1.0 / x;
+#endif
+  }
+  const double y0 = dbl_from(ff_rcpf(ff_lead(x)));
+  const double e = fma(-x, y0, 1.0);
+  return fma(y0, fma(e, e, e), y0);
+}
+
 // Largest relative jump that takes the pair path.
 constexpr float kRoeJump = 0.00390625f;  // 2^-8
 
@@ -237,8 +254,7 @@ DG_HD void roe_flux2_small(const double qm[4], const double qp[4], const double 
   const ff dr = ff_from(qp[0] - qm[0]), da = ff_from(qp[1] - qm[1]), db = ff_from(qp[2] - qm[2]),
            de = ff_from(qp[3] - qm[3]);
   const ff rL = ff_from(qm[0]), rR = ff_from(qp[0]);
-  // 1 / rho of both sides from one reciprocal of the product: a float seed, corrected by
-  // y (1 + e + e^2), e = 1 - x y (e < 2^-21: the cut term is below 2^-63)
+  // 1 / rho of both sides from one reciprocal of the product (in 2^-60 .. 2^60; as rcp_seeded)
   const double x = qm[0] * qp[0];
   const double y0 = dbl_from(ff_rcpf(ff_lead(x)));
   const double e0 = fma(-x, y0, 1.0);

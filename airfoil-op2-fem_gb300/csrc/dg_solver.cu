@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(32 * np_of(N)) elem_kernel(const Inst d, const
     const double rx = g[0], ry = g[1], sx = g[2], sy = g[3];
     double fr0 = 0, fr1 = 0, fr2 = 0, fr3 = 0, fs0 = 0, fs1 = 0, fs2 = 0, fs3 = 0;
     if (live) {
-      const double ir = rcp(w[0]);
+      const double ir = rcp_seeded(w[0]);
       const double u = w[1] * ir, v = w[2] * ir;
       const double p = P.gm1 * fma(-0.5, fma(w[1], u, w[2] * v), w[3]);
       const double ep = w[3] + p;
@@ -498,7 +498,7 @@ __device__ __forceinline__ void elem_tile_sym(const Inst &d, const int stage, co
     const double rx = g[0], ry = g[1], sx = g[2], sy = g[3];
     double fr0 = 0, fr1 = 0, fr2 = 0, fr3 = 0, fs0 = 0, fs1 = 0, fs2 = 0, fs3 = 0;
     if (live) {
-      const double ir = rcp(w[0]);
+      const double ir = rcp_seeded(w[0]);
       const double u = w[1] * ir, v = w[2] * ir;
       const double p = P.gm1 * fma(-0.5, fma(w[1], u, w[2] * v), w[3]);
       const double ep = w[3] + p;
