@@ -365,28 +365,28 @@ __global__ void k_zero(long long n, double *p) {
   if (t < n) p[t] = 0.0;
 }
 
-// src/calc_dt.h:3-22, the OP_MAX combined on the bit patterns of non-negative doubles
+// src/calc_dt.h:3-22, the OP_MAX combined on the bit patterns of non-negative doubles; one thread per face
+// point (one per cell: 69 us for K = 32768, N = 3 with the copy of the result, now 63)
 template <int N>
 __global__ void k_calc_dt(int n, const double *q, const double *fscale, double seed,
                           unsigned long long *red, const Consts C) {
   constexpr int Np = Ord<N>::Np, Nfp = Ord<N>::Nfp;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   double max = seed;
-  if (c < n) {
+  if (t < (long long)n * 3 * Nfp) {
+    const int c = (int)(t / (3 * Nfp)), i = (int)(t - (long long)c * (3 * Nfp));
     const double *qc = q + (size_t)4 * Np * c;
     const double *fs = fscale + (size_t)3 * Nfp * c;
-    const int *F = C.FMASK;
+    const int F = C.FMASK[i];
     const double gam = C.gam;
-    for (int i = 0; i < 3 * Nfp; i++) {
-      double rho = qc[F[i] * 4];
-      double u = qc[F[i] * 4 + 1] / rho;
-      double v = qc[F[i] * 4 + 2] / rho;
-      double p = (gam - 1.0) * (qc[F[i] * 4 + 3] - rho * (u * u + v * v) * 0.5);
-      double cs = sqrt(fabs(gam * p / rho));
-      const int fi = (Np <= 3 * Nfp) ? F[i] : i;
-      double val = ((N + 1) * (N + 1)) * 0.5 * fs[fi] * (sqrt(u * u + v * v) + cs);
-      if (val > max) max = val;
-    }
+    double rho = qc[F * 4];
+    double u = qc[F * 4 + 1] / rho;
+    double v = qc[F * 4 + 2] / rho;
+    double p = (gam - 1.0) * (qc[F * 4 + 3] - rho * (u * u + v * v) * 0.5);
+    double cs = sqrt(fabs(gam * p / rho));
+    const int fi = (Np <= 3 * Nfp) ? F : i;
+    double val = ((N + 1) * (N + 1)) * 0.5 * fs[fi] * (sqrt(u * u + v * v) + cs);
+    if (val > max) max = val;
   }
   unsigned long long b = max > 0.0 ? (unsigned long long)__double_as_longlong(max) : 0ull;
   for (int o = 16; o > 0; o >>= 1) {
@@ -582,12 +582,31 @@ __global__ void k_set_workingQ(long long n, double dt, int stage, const double *
   else W[i] = q[i] + dt * (k1[i] / 4.0 + k2[i] / 4.0);
 }
 
+// x / B rounded to nearest for B = 3 or 6, in three FP64 instructions (a division takes ten and more, and
+// update_Q below was bound by them: 87 -> 60 us for K = 32768, N = 3).  With y the double
+// nearest to 1 / B and x in the range below: q = x y is within two units in the last place of x / B, so
+// the remainder r = x - B q (a small multiple of q's last place) is exact and q + r y differs from
+// x / B by less than 2^-51 of that place before its one rounding; x / B is at least 1/6 of it away from
+// any midpoint (X 2^m - B (odd) is no smaller than 1 for B = 3, 2 for B = 6, over 2 B).  Zero keeps its
+// sign; the rest (near the ends of the exponent range, non-finite) is divided.
+template <int B>
+__device__ __forceinline__ double div_exact(const double x) {
+  static_assert(B == 3 || B == 6, "the margin above is for 3 and 6");
+  constexpr double y = 1.0 / B;
+  const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7FFu;
+  if (e - 100u < 1900u) {
+    const double q = __dmul_rn(x, y);
+    return __fma_rn(__fma_rn(-(double)B, q, x), y, q);
+  }
+  return (__double_as_longlong(x) << 1) == 0 ? x : x / (double)B;
+}
+
 // src/update_Q.h:1-12, one thread per value
 __global__ void k_update_Q(long long n, double dt, double *q, const double *k1, const double *k2,
                            const double *k3, double *W) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  q[i] = q[i] + dt * (k1[i] / 6.0 + k2[i] / 6.0 + 2.0 * k3[i] / 3.0);
+  q[i] = q[i] + dt * (div_exact<6>(k1[i]) + div_exact<6>(k2[i]) + div_exact<3>(2.0 * k3[i]));
   W[i] = q[i];
 }
 
@@ -698,26 +717,65 @@ T *dptr(const op_arg &a) {
   return (T *)a.dat->d_data;
 }
 
+// Device time of each loop: a pair of events around its launch, read later.  The loops run in stream
+// order without waiting for one another; only what hands a value to the host waits (calc_dt's and
+// l2_error's reductions, op_fetch_data), and there the finished pairs are read.  A wait after every
+// loop left the GPU idle for a launch and a host round trip 13 times a step.
+struct TimedPair {
+  cudaEvent_t a, b;
+  LoopStat *stat;
+};
+struct TimerPool {
+  std::vector<TimedPair> pending;
+  std::vector<cudaEvent_t> idle;
+  cudaEvent_t take() {
+    cudaEvent_t e = nullptr;
+    if (!idle.empty()) {
+      e = idle.back();
+      idle.pop_back();
+    } else {
+      cudaEventCreate(&e);
+    }
+    return e;
+  }
+};
+TimerPool &TP() {
+  static TimerPool p;
+  return p;
+}
+
+// Reads every pending pair (waits for the last of them) and returns its events to the pool.
+void read_timers() {
+  TimerPool &p = TP();
+  if (p.pending.empty()) return;
+  cudaEventSynchronize(p.pending.back().b);  // one stream: the earlier ones are done too
+  for (TimedPair &t : p.pending) {
+    float ms = 0;
+    if (cudaEventElapsedTime(&ms, t.a, t.b) == cudaSuccess) t.stat->ms += ms;
+    t.stat->count++;
+    p.idle.push_back(t.a);
+    p.idle.push_back(t.b);
+  }
+  p.pending.clear();
+}
+
 struct Timed {
   cudaEvent_t a = nullptr, b = nullptr;
-  std::string name;
-  explicit Timed(const char *n) : name(n) {
-    cudaEventCreate(&a);
-    cudaEventCreate(&b);
+  LoopStat *stat;
+  explicit Timed(const char *n) : stat(&S().stats[n]) {  // map nodes keep their address
+    a = TP().take();
+    b = TP().take();
     cudaEventRecord(a, S().stream);
   }
   void done() {
     cudaEventRecord(b, S().stream);
-    cudaEventSynchronize(b);  // loops are short; timing every one matches op_timers in the driver
-    float ms = 0;
-    cudaEventElapsedTime(&ms, a, b);
-    LoopStat &st = S().stats[name];
-    st.count++;
-    st.ms += ms;
+    TP().pending.push_back(TimedPair{a, b, stat});
+    a = b = nullptr;
+    if (TP().pending.size() >= 1024) read_timers();  // an application that never reads a value back
   }
-  ~Timed() {
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
+  ~Timed() {  // a launch failed: nothing was timed
+    if (a) TP().idle.push_back(a);
+    if (b) TP().idle.push_back(b);
   }
 };
 
@@ -746,6 +804,7 @@ int op2_gb300_sync(void) {
 void op2_gb300_reset(void) {
   State &s = S();
   if (s.stream) cudaStreamSynchronize(s.stream);
+  read_timers();
   for (auto &m : s.maps) cudaFree(m->d_data);
   for (auto &d : s.dats) cudaFree(d->d_data);
   for (auto &c : s.consts) cudaFree(c.second.second);
@@ -828,7 +887,10 @@ void op_decl_const2(char const *name, int dim, char const *type, void *data) {
   if (!ensure_stream()) return;
   const size_t bytes = (size_t)dim * (dbl ? 8 : 4);
   auto &slot = S().consts[name];
-  if (slot.second) cudaFree(slot.second);
+  if (slot.second) {
+    cudaStreamSynchronize(S().stream);  // loops still running may read the old values
+    cudaFree(slot.second);
+  }
   slot.first.assign((const char *)data, (const char *)data + bytes);
   slot.second = nullptr;
   if (!ck(cudaMalloc(&slot.second, bytes), "cudaMalloc")) return;
@@ -866,7 +928,7 @@ void op_fetch_data(op_dat dat, void *data) {
   if (!dat || !data) { fail("op_fetch_data: bad arguments"); return; }
   const size_t bytes = (size_t)dat->set->size * dat->dim * (dat->is_double ? 8 : 4);
   if (!ck(cudaMemcpyAsync(data, dat->d_data, bytes, cudaMemcpyDeviceToHost, S().stream), "cudaMemcpyAsync")) return;
-  ck(cudaStreamSynchronize(S().stream), "cudaStreamSynchronize");
+  if (ck(cudaStreamSynchronize(S().stream), "cudaStreamSynchronize")) read_timers();
 }
 
 int op_get_size(op_set set) { return set ? set->size : 0; }
@@ -879,9 +941,10 @@ void op_timers(double *cpu, double *wall) {
 }
 
 void op_timing_output(void) {
+  read_timers();
   printf("\n  count   device time (ms)   kernel\n");
   for (auto &kv : S().stats)
-    printf(" %6d  %16.4f   %s\n", kv.second.count, kv.second.ms, kv.first.c_str());
+    if (kv.second.count) printf(" %6d  %16.4f   %s\n", kv.second.count, kv.second.ms, kv.first.c_str());
 }
 
 // ------------------------------------------------------------------ loops
@@ -961,7 +1024,7 @@ void op_par_loop_calc_dt(char const *name, op_set set, op_arg a0, op_arg a1, op_
   std::memcpy(&seed, a2.data, 8);
   unsigned long long seed_bits = seed > 0.0 ? (unsigned long long)__builtin_bit_cast(long long, seed) : 0ull;
   if (!ck(cudaMemcpyAsync(S().d_red, &seed_bits, 8, cudaMemcpyHostToDevice, S().stream), "cudaMemcpyAsync")) return;
-  DISPATCH_N(N, (k_calc_dt<N><<<blocks(set->size, 128), 128, 0, S().stream>>>(
+  DISPATCH_N(N, (k_calc_dt<N><<<blocks((long long)set->size * 3 * (N + 1), 128), 128, 0, S().stream>>>(
                     set->size, dptr<double>(a0), dptr<double>(a1), seed, (unsigned long long *)S().d_red, C)));
   if (!ck(cudaGetLastError(), "calc_dt launch")) return;
   unsigned long long bits = 0;
@@ -972,6 +1035,7 @@ void op_par_loop_calc_dt(char const *name, op_set set, op_arg a0, op_arg a1, op_
   if (seed > out) out = seed;
   std::memcpy(a2.data, &out, 8);
   t.done();
+  read_timers();
 }
 
 // src/airfoil.cpp:256-265
