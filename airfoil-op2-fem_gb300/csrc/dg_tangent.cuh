@@ -387,6 +387,7 @@ inline int adjoint_tangent(Adjoint &A, double dpar, const double *dq0_host, doub
   if (!A.have_forward) { err = "call forward first"; return -1; }
   Solver &s = *A.fwd;
   cudaStream_t st = s.stream;
+  A.seg_last = false;  // this run moves the solver's state
   if (int rc = s.init(err)) return rc;
   s.d.dt_mode = 1;
   const int N = A.cfg.N;
