@@ -321,6 +321,22 @@ __global__ void advec_coef_kernel(const AdvInst d, double *coef) {
   }
 }
 
+// AdvInst::nbr from the edge records, a thread per edge; every cell face has exactly one edge
+// (validate), so every entry is written once.  (Built on the host and copied, set-up took 2 ms more at
+// K = 524288.)
+__global__ void advec_nbr_kernel(const AdvInst d, int2 *nbr) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < d.nE) {
+    const int4 e = d.edges[k];
+    const int fL = e.z & 3, fR = (e.z >> 2) & 3, rev = (e.z >> 4) & 1;
+    nbr[3 * (size_t)e.x + fL] = make_int2(e.y, fR | (rev << 2));
+    nbr[3 * (size_t)e.y + fR] = make_int2(e.x, fL | (rev << 2));
+  } else if (k - d.nE < d.nB) {
+    const int4 b = d.bedges[k - d.nE];
+    nbr[3 * (size_t)b.x + b.y] = make_int2(-1, 0);
+  }
+}
+
 // advec/src/set_ic.h:3-10 at the node positions of src/init_grid.h.
 template <int N>
 __global__ void advec_ic_kernel(const AdvInst d, const double *coords, const int *cells) {
@@ -450,12 +466,6 @@ int Advection::create(const Mesh &m, int order, double vel_x, double vel_y, doub
   d.coef = coef;
   int2 *nbr = (int2 *)alloc((size_t)K * 3 * sizeof(int2));
   d.nbr = nbr;
-  std::vector<int2> nb((size_t)K * 3, make_int2(-1, 0));
-  for (const int4 &e : edges) {
-    const int fL = e.z & 3, fR = (e.z >> 2) & 3, rev = (e.z >> 4) & 1;
-    nb[3 * (size_t)e.x + fL] = make_int2(e.y, fR | (rev << 2));
-    nb[3 * (size_t)e.y + fR] = make_int2(e.x, fL | (rev << 2));
-  }
   int4 *de = (int4 *)alloc(sizeof(int4) * d.nE), *db = (int4 *)alloc(sizeof(int4) * d.nB);
   d.edges = de;
   d.bedges = db;
@@ -474,9 +484,9 @@ int Advection::create(const Mesh &m, int order, double vel_x, double vel_y, doub
   CK(cudaMemcpyAsync(cells_d, m.cell2nodes.data(), m.cell2nodes.size() * 4, cudaMemcpyHostToDevice, stream));
   CK(cudaMemsetAsync(d.flux, 0, (size_t)K * 3 * Nfp * 8, stream));
   CK(cudaMemsetAsync(d.acc, 0, nq * 8, stream));
-  CK(cudaMemcpyAsync(nbr, nb.data(), nb.size() * sizeof(int2), cudaMemcpyHostToDevice, stream));
   geometry_kernel<<<(K + 127) / 128, 128, 0, stream>>>(K, coords_d, cells_d, geo);
   advec_coef_kernel<<<(K + 127) / 128, 128, 0, stream>>>(d, coef);
+  advec_nbr_kernel<<<(d.nE + d.nB + 127) / 128, 128, 0, stream>>>(d, nbr);
   CK(cudaGetLastError());
   DG_DISPATCH(N, CK(cudaFuncSetAttribute(advec_fused_kernel<NN, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)advec_fused_smem<NN>(128))));  // 16 cells need 16 KB at most
