@@ -407,7 +407,7 @@ class Solver:
 
 
 class Batch:
-    """Many instances advanced together by one persistent kernel per RK stage (dg_batch_t)."""
+    """Many instances advanced together by shared launches per RK stage (dg_batch_t)."""
 
     def __init__(self, meshes, cfgs):
         assert len(meshes) == len(cfgs) and meshes

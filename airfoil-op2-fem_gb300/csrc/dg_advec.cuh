@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(32 * np_of(N)) advec_elem_kernel_sym(const Adv
 //      a face kernel's flux array (a write and a read of 3 Nfp values per cell and stage) and its
 //      launch are not needed, at the price of reading W of one buffer and writing another.
 //   2. operand pre-pass, contraction, 3. recombination and the RK4 combine of advec_elem_kernel.
-// ~120 FP64 instructions per cell at N = 4 (100 us of the 260 us stage at K = 524288); the rest is the
+// 121-134 FP64 instructions per cell at N = 4 (116-127 us of the 256-261 us stage at K = 524288); the rest is the
 // integer work of the exact product.  Step at K = 524288, N = 1 / 2 / 3 / 4: 404 / 800 / 1083 / 2449 ->
 // 283 / 461 / 716 / 1039 us; K = 259200, N = 5 / 6: 1960 / 3093 -> 952 / 1231 us (before: a face kernel and
 // an element kernel in FP64, on the tensor cores at N = 3).

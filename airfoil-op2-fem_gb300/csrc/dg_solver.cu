@@ -7,13 +7,14 @@
 //                (src/euler_rhs.h:120-220) and writes twice it (the 1/2 is in the LIFT
 //                columns), scaled by each side's fscale, into both cells' face slots.  Each
 //                slot has exactly one writer: no atomics.
-//   elem_kernel  32 cells x Np node-warps per block: nodal Euler fluxes combined with the
-//                (affine, per-cell) metric terms, one contraction of [Drw | Dsw | -LIFT/2]
-//                (operators in constant memory, warp-uniform rows) against
+//   elem_kernel  a tile of cells per block (32, or 8 / 16 where elem_small() says so), one thread
+//                per cell and node: nodal Euler fluxes combined with the (affine, per-cell)
+//                metric terms, one contraction of [Drw | Dsw | -LIFT/2] against
 //                [Fr ; Fs ; flux] staged in shared memory (src/euler_rhs.h:226-247,284-286),
+//                on the tensor cores as an exact integer product (dg_ozaki.cuh),
 //                then the SSPRK3 stage combine in registers (src/set_workingQ.h,
 //                src/update_Q.h, in Shu-Osher form) and, in the last stage, single-precision
-//                calc_dt estimates (src/calc_dt.h) on the new state, one maximum per node-warp.
+//                calc_dt estimates (src/calc_dt.h) on the new state, one maximum per 8 cells.
 // plus a finalize kernel per step: the exact FP64 calc_dt maximum over the candidate nodes the
 // estimates single out (dt_finalize_kernel), then t += dt; dt = (1/dt1)*cfl.  dt never leaves the
 // device, so a whole step is a fixed launch sequence that is captured once in a CUDA graph.
@@ -222,9 +223,9 @@ __global__ void __launch_bounds__(256) face_kernel(const Inst d, const int stage
   face_node<N, true>(d, stage, tid);
 }
 
-// The same in 64-thread blocks compiled for 16 resident blocks per SM (at most 64 registers):
-// one such block fits on an SM beside three order-3 element blocks (3 x 20,480 + 4,096 = 65,536
-// registers), so face blocks of one cell range can run next to element blocks of another.
+// The same in 64-thread blocks compiled for 16 resident blocks per SM: at most 64 registers whatever
+// the compiler takes for the launch above (64 at N = 3), so that one block fits on an SM beside three
+// order-3 element blocks (3 x 20,480 + 4,096 = 65,536 registers).
 template <int N>
 __global__ void __launch_bounds__(64, 16) face_kernel_r64(const Inst d, const int stage) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -263,8 +264,8 @@ __device__ __forceinline__ unsigned long long dt_speed_bits(const double n0, con
   return (unsigned long long)__double_as_longlong(spd * fs);
 }
 
-// SSPRK3 stage combine of one node's right-hand side (r0..r3), and in the last stage each
-// node-warp's largest single-precision calc_dt estimate (Inst::dt_est; the step's finalize takes
+// SSPRK3 stage combine of one node's right-hand side (r0..r3), and in the last stage the
+// largest single-precision calc_dt estimate of the node in each 8 cells (Inst::dt_est; the step's finalize takes
 // the FP64 maximum).  Every thread of the node-warps calls it: `active` is false for warps beyond
 // the Np node-warps of a wider block, `live` is false for lanes past the last cell (they take part
 // in the warp reductions).  qs: this node's q staged in shared memory (qs[0] variables 0, 1 and
@@ -333,8 +334,8 @@ __device__ __forceinline__ void stage_combine(const Inst &d, const int stage, co
     // src/calc_dt.h: (N+1)^2 * 0.5 * fscale * (|v| + c) at the face points of this node, maximised
     // over the mesh.  Here only a single-precision estimate (from bit-truncated copies of the
     // state, f32_trunc, and single-precision copies of fscale and gamma), within ~1e-6 of the FP64
-    // value: each node-warp stores its largest estimate and combines it into the step state's
-    // maximum estimate; the step's finalize (dt_finalize_kernel, batch_dt_finalize_kernel)
+    // value: the largest one of the node in each 8 cells (kDtCells) is stored and combined into the
+    // step state's maximum estimate; the step's finalize (dt_finalize_kernel, batch_dt_finalize_kernel)
     // evaluates in FP64 the nodes whose estimate is within 1e-4 of that maximum, among them the
     // node of the FP64 maximum.  No barrier and no FP64 instruction here: evaluating a block's
     // candidates in this kernel (a barrier, a ~35-long FP64 chain waiting behind the other blocks'
@@ -670,12 +671,10 @@ __global__ void finalize_kernel(StepState *st, int dt_mode, double *dt_hist, uns
 }
 
 // The per-step finalize with the deferred calc_dt maximum (Inst::dt_est): with M the largest
-// single-precision estimate of the mesh (the element kernel's node-warps combine theirs into the
-// step state by atomicMax), the grid's warps share the node-warps whose estimate is within 1e-4
-// of M and evaluate those
-// nodes in FP64 from the new q (the estimates are within ~1e-6 of the FP64 values, so the node
-// of the FP64 maximum is always among them and the result is the exact maximum, the same as the
-// element kernel's per-block evaluation gives), combined with atomicMax; the last block to finish
+// single-precision estimate of the mesh (the element kernel combines its own into the step state by
+// atomicMax), the grid's warps share the estimates (each of one node in 8 cells) within 1e-4 of M
+// and evaluate those nodes in FP64 from the new q (the estimates are within ~1e-6 of the FP64 values, so the node
+// of the FP64 maximum is always among them and the result is the exact maximum), combined with atomicMax; the last block to finish
 // (a counter in the step state, no waiting) then advances t and sets the new dt.
 // calc_dt of node i of cell e (src/calc_dt.h) in FP64 from q, as the bit pattern of a non-negative
 // double; 0 for a cell past the last or a node without face points.
@@ -954,11 +953,11 @@ __global__ void vertex_fields_kernel(int K, const int *cells, const int *owner, 
 }
 
 // ---------------------------------------------------------------- launch helpers
-// Threads per face-kernel block (a multiple of 32, at most 256).  The 68-register face blocks
-// fill an SM with ~30 warps; with 256-thread blocks the last of ~1.7 waves leaves SMs idle
-// (SM active 70 % of the launch).  Small blocks let the block scheduler balance that tail:
-// 64 threads measured 58.5 / 61.8 us per stage at N=3 / N=4 on the K=32768 O-grid against
-// 65.9 / 74.0 us with 256.
+// Threads per face-kernel block (a multiple of 32, at most 256).  Small
+// blocks let the block scheduler balance the launch's tail, which matters most where a launch is
+// one or two waves: steps of the K=32768 O-grid with blocks of 32 / 64 / 128 / 256 threads 116.1 /
+// 116.2 / 117.2 / 123.7 us at N=2, 181.0 / 181.7 / 184.4 / 182.6 at N=3, 438.9 / 438.7 / 438.9 /
+// 439.3 at N=5; no difference above 0.1 % at K=131072.
 static std::atomic<int> g_face_block{64};
 // 1: 64-thread face blocks use face_kernel_r64 (at most 64 registers).
 static std::atomic<int> g_face_r64{0};
@@ -1648,8 +1647,11 @@ int step_graph_flags() { return g_step_graph_flags; }
 int step_parts_for(int K) {
   const int T = (K + 31) / 32, sp = g_step_parts.load();
   if (sp >= 1) return std::max(1, std::min(sp, std::min(kMaxStepParts, T)));
-  // automatic: ranges of at least 128 tiles, at most 4 (on the K = 32768 O-grid at N = 3, steps of
-  // 290 / 267 / 269 / 271 us with 1 / 4 / 8 / 16 ranges; more ranges add launches and edges)
+  // automatic: ranges of at least 128 tiles, at most 4.  Steps in runs with 1 / 2 / 4 / 8 ranges: K =
+  // 32768 202.4 / 201.0 / 181.6 / 176.3 us at N = 3, 320.8 / 309.9 / 292.1 / 290.0 at N = 4; K = 131072
+  // 717 / 686 / 671 / 676 at N = 3.  More ranges and smaller meshes gain in long runs (K = 7168, N = 3
+  // with 1 / 2 ranges 89.4 / 70.0), but the longer capture takes ~110 us of a solver's first call (one
+  // step of K = 7168 138 -> 261 us).
   return std::max(1, std::min(4, T / 128));
 }
 
