@@ -711,7 +711,7 @@ int dg_roe_pair_flux(double gam, int n, const double *qm, const double *qp, cons
   P.rinf = P.pinf = 1.0;
   P.derive();
   for (int k = 0; k < n; k++) {
-    taken[k] = dg::roe_small_jump(qm + 4 * k, qp + 4 * k) ? 1 : 0;
+    taken[k] = dg::roe_small_jump(qm + 4 * k, qp + 4 * k, P.gm1f) ? 1 : 0;
     for (int j = 0; j < 4; j++) f2[4 * k + j] = 0.0;
     if (taken[k])
       dg::roe_flux2_small(qm + 4 * k, qp + 4 * k, nrm[2 * k], nrm[2 * k + 1], P.gm1, dg::ff{P.gm1f, P.gm1l}, f2 + 4 * k);

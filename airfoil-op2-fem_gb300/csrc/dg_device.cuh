@@ -118,7 +118,7 @@ __device__ __forceinline__ void roe_flux2(const double qm[4], const double qp[4]
 // warp with nodes of both kinds runs both.
 __device__ __forceinline__ void roe_flux2_face(const double qm[4], const double qp[4], const double nx,
                                                const double ny, const Phys &P, double f2[4]) {
-  if (roe_small_jump(qm, qp)) roe_flux2_small(qm, qp, nx, ny, P.gm1, ff{P.gm1f, P.gm1l}, f2);
+  if (roe_small_jump(qm, qp, P.gm1f)) roe_flux2_small(qm, qp, nx, ny, P.gm1, ff{P.gm1f, P.gm1l}, f2);
   else roe_flux2(qm, qp, nx, ny, P, f2);
 }
 

@@ -12,19 +12,30 @@
 //
 // Measured (stage launches alone, GB300): K = 32768 O-grid, N = 3 49.5 -> 28.5 us; K = 18990,
 // N = 5 41 -> 26.6 us; K = 524288 square, N = 4 790 -> 404 us (FP64 floors at 109 and 53
-// instructions: 34 / 17, 30 / 15 and 683 / 332 us).  Against 113-bit arithmetic the flux's error
-// (random states, jumps up to the line) is 0.33-0.58 units of 2^-53 rms per component, where
-// roe_flux2 has 0.50-0.83.  The line lies at 2^-8: at 2^-7 the momentum components' rms is 4 %
-// above roe_flux2's, and above a Mach number of about 4 the largest errors double.
+// instructions: 34 / 17, 30 / 15 and 683 / 332 us).
+//
+// Accuracy.  Against 113-bit arithmetic, random states at Mach numbers to 0.1, 0.8 and 1.9, the
+// components' errors at jumps up to the line, in units of 2^-53 of the flux's scale, rms (roe_flux2's
+// in brackets): gamma = 1.4 0.11-0.77 (0.54-0.84), 0.28-0.52 (0.46-0.71), 0.43-0.59 (0.56-0.95); no
+// component's rms is above roe_flux2's from gamma = 1.00001 to 8 (with the seeds below moved by a unit
+// (reciprocal) or two (root) in the last place as the hardware's are).  Three things make it so:
+//   - the seeds are refined to second order: with one correction e of 2^-22 cut at e^2, the roots
+//     and reciprocals were known to 2^-44 only (momentum 1.04 rms at jumps up to the line);
+//   - the halves of a dissipation component are joined in FP64 before they are subtracted, one
+//     rounding at the flux's full size less (the pressure term added last would save another, but
+//     takes 77 registers instead of 64: vortex steps of K = 2048 10 % and of K = 524288 2 % slower);
+//   - the rule below measures jumps and Mach numbers by the sound speed, not by sqrt(E / rho), which
+//     is far above it as gamma nears 1 (errors of 30 units there).
 //
 // roe_small_jump decides per face node, from the states alone (so every launch form gives a node
-// the same path): jumps of rho, rho (u, v) and E below 2^-8 of rho, sqrt(rho E) and E, both sides
-// physical with a Mach number below about 1.9, and magnitudes for which no float over- or
-// underflows.  Everything else (strong jumps, non-finite or non-physical states, extreme
-// scales) takes roe_flux2.
+// the same path): jumps of rho, rho (u, v) and E below 2^-8 of rho, sqrt(g rho E) and E, both sides
+// physical with |rho (u, v)|^2 below g rho E, g = min(1, 5 (gamma - 1) / 2) (at gamma = 1.4 a Mach
+// number below 1.9, at 1.01 below 1.6), and magnitudes for which no float over- or underflows.
+// Everything else (strong jumps, non-finite or non-physical states, extreme scales) takes roe_flux2.
 //
 // Pair arithmetic after Dekker, "A floating-point technique for extending the available
-// precision", Numer. Math. 18 (1971), with fused multiply-adds for the product's error.
+// precision", Numer. Math. 18 (1971), the sums by Knuth's six-operation form (The Art of Computer
+// Programming, vol. 2, 4.2.2), with fused multiply-adds for the product's error.
 #pragma once
 #include <cmath>
 #include <cstdint>
@@ -153,15 +164,17 @@ DG_HD ff ff_fma(const ff a, const ff b, const ff c) {
   return ff_norm(s, ff_addf(d, ff_addf(e, c.l)));
 }
 DG_HD ff ff_half(const ff a) { return ff{ff_mulf(0.5f, a.h), ff_mulf(0.5f, a.l)}; }
-// 1 / a, from a single-precision reciprocal and one correction (residual by fused multiply-adds)
+// 1 / a, from a single-precision reciprocal y: y (1 + e + e^2), e = 1 - a y by fused multiply-adds
 DG_HD ff ff_rcp(const ff a) {
   const float y = ff_rcpf(a.h);
   const float e = ff_fmaf(-a.l, y, ff_fmaf(-a.h, y, 1.0f));
-  return ff_norm(y, ff_mulf(y, e));
+  return ff_norm(y, ff_mulf(y, ff_fmaf(e, e, e)));
 }
-// sqrt(a) for a > 0: s = a y with y ~ 1 / sqrt(a), corrected by (a - s^2) y / 2
+// sqrt(a) for a > 0: y ~ 1 / sqrt(a) after one Newton step in single precision, s = a y, corrected
+// by (a - s^2) y / 2
 DG_HD ff ff_sqrt(const ff a) {
-  const float y = ff_rsqrtf(a.h);
+  const float y0 = ff_rsqrtf(a.h), s0 = ff_mulf(a.h, y0);
+  const float y = ff_fmaf(ff_mulf(0.5f, y0), ff_fmaf(-s0, y0, 1.0f), y0);
   const float s = ff_mulf(a.h, y);
   const float r = ff_addf(ff_fmaf(-s, s, a.h), a.l);
   return ff_norm(s, ff_mulf(ff_mulf(0.5f, y), r));
@@ -215,8 +228,9 @@ DG_HD double rcp_seeded(const double x) {
 // Largest relative jump that takes the pair path.
 constexpr float kRoeJump = 0.00390625f;  // 2^-8
 
-// Whether roe_flux2_small may take this face node (see the head of this file).
-DG_HD bool roe_small_jump(const double qm[4], const double qp[4]) {
+// Whether roe_flux2_small may take this face node (see the head of this file); gm1: gamma - 1.  Written in
+// single rounded operations, so that every kernel decides alike.
+DG_HD bool roe_small_jump(const double qm[4], const double qp[4], const float gm1) {
   // rho and E of both sides positive, in 2^-30 .. 2^30; momenta below 2^60 (the float squares
   // below stay finite, the conversions in range)
   const uint32_t lim = 60u << 20, off = (1023u - 30u) << 20;
@@ -230,10 +244,14 @@ DG_HD bool roe_small_jump(const double qm[4], const double qp[4]) {
   const float rL = ff_lead(qm[0]), aL = ff_lead(qm[1]), bL = ff_lead(qm[2]), eL = ff_lead(qm[3]);
   const float rR = ff_lead(qp[0]), aR = ff_lead(qp[1]), bR = ff_lead(qp[2]), eR = ff_lead(qp[3]);
   const float rmin = rL < rR ? rL : rR, emin = eL < eR ? eL : eR;
-  const float dr = std::fabs(rL - rR), de = std::fabs(eL - eR), da = aL - aR, db = bL - bR;
-  const float reL = rL * eL, reR = rR * eR;
-  return (dr <= kRoeJump * rmin) & (de <= kRoeJump * emin) & (da * da + db * db <= (kRoeJump * kRoeJump) * (rmin * emin)) &
-         (aL * aL + bL * bL <= reL) & (aR * aR + bR * bR <= reR);
+  const float dr = std::fabs(ff_addf(rL, -rR)), de = std::fabs(ff_addf(eL, -eR)), da = ff_addf(aL, -aR),
+              db = ff_addf(bL, -bR);
+  const float g25 = ff_mulf(2.5f, gm1), g = g25 < 1.0f ? g25 : 1.0f;
+  const float jm = ff_mulf(kRoeJump * kRoeJump, ff_mulf(g, ff_mulf(rmin, emin)));
+  return (dr <= ff_mulf(kRoeJump, rmin)) & (de <= ff_mulf(kRoeJump, emin)) &
+         (ff_fmaf(da, da, ff_mulf(db, db)) <= jm) &
+         (ff_fmaf(aL, aL, ff_mulf(bL, bL)) <= ff_mulf(g, ff_mulf(rL, eL))) &
+         (ff_fmaf(aR, aR, ff_mulf(bR, bR)) <= ff_mulf(g, ff_mulf(rR, eR)));
 }
 
 // Twice the Roe flux (as roe_flux2) of a face node that roe_small_jump accepts.  gm1, gf: gamma - 1
@@ -266,11 +284,9 @@ DG_HD void roe_flux2_small(const double qm[4], const double qp[4], const double 
   const double kL = fma(-0.5, fma(qm[1], qm[1], qm[2] * qm[2]) * irL, qm[3]);  // p / (gamma - 1)
   const double kR = fma(-0.5, fma(qp[1], qp[1], qp[2] * qp[2]) * irR, qp[3]);
   const double EL = fma(gm1, kL, qm[3]), ER = fma(gm1, kR, qp[3]);  // E + p
-  const double ps = gm1 * (kL + kR);
-  double f0 = mL + mR;
-  double f1 = fma(nx, ps, fma(qm[1], uL, qp[1] * uR));
-  double f2y = fma(ny, ps, fma(qm[2], uL, qp[2] * uR));
-  double f3 = fma(uL, EL, uR * ER);
+  const double ps = fma(gm1, kL, gm1 * kR);
+  const double f0 = mL + mR, f1 = fma(nx, ps, fma(qm[1], uL, qp[1] * uR)), f2y = fma(ny, ps, fma(qm[2], uL, qp[2] * uR)),
+               f3 = fma(uL, EL, uR * ER);
   // Roe averages in pairs: x = wL (rho x)_L + wR (rho x)_R, wL = 1 / (rho_L + g), wR = 1 / (rho_R + g),
   // g = sqrt(rho_L rho_R)
   const ff g = ff_sqrt(ff_mul(rL, rR));
@@ -304,10 +320,10 @@ DG_HD void roe_flux2_small(const double qm[4], const double qp[4], const double 
   const ff d1 = ff_fma(u, d0, ff_fma(nxf, ce, ff_mul(au, sa)));
   const ff d2 = ff_fma(v, d0, ff_fma(nyf, ce, ff_mul(au, sb)));
   const ff d3 = ff_fma(H, d14, ff_fma(un, ce, ff_fma(q2, W2, ff_mul(au, us))));
-  f2[0] = (f0 - dbl_from(d0.h)) - dbl_from(d0.l);
-  f2[1] = (f1 - dbl_from(d1.h)) - dbl_from(d1.l);
-  f2[2] = (f2y - dbl_from(d2.h)) - dbl_from(d2.l);
-  f2[3] = (f3 - dbl_from(d3.h)) - dbl_from(d3.l);
+  f2[0] = f0 - (dbl_from(d0.h) + dbl_from(d0.l));
+  f2[1] = f1 - (dbl_from(d1.h) + dbl_from(d1.l));
+  f2[2] = f2y - (dbl_from(d2.h) + dbl_from(d2.l));
+  f2[3] = f3 - (dbl_from(d3.h) + dbl_from(d3.l));
 }
 
 }  // namespace dg

@@ -2206,6 +2206,53 @@ extern "C" int dg_boundary_state(const dg_config_t *cfg, int type, int n, const 
   return 0;
 }
 
+// ---------------------------------------------------------------- Roe flux of given states
+// dg_roe_flux_nodes (include/dg_gb300.h): the face kernels' flux functions applied to n given pairs of
+// states, so that tests can measure their rounding on the device, whose seeds the host copy
+// (dg_roe_pair_flux) does not have.
+namespace dg {
+__global__ void roe_flux_kernel(int n, int form, const double *qm, const double *qp, const double *nrm, Phys P, double *f2) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  double a[4], b[4], f[4];
+  for (int j = 0; j < 4; j++) {
+    a[j] = qm[4 * k + j];
+    b[j] = qp[4 * k + j];
+  }
+  if (form == 0) roe_flux2(a, b, nrm[2 * k], nrm[2 * k + 1], P, f);
+  else roe_flux2_face(a, b, nrm[2 * k], nrm[2 * k + 1], P, f);
+  for (int j = 0; j < 4; j++) f2[4 * k + j] = f[j];
+}
+}  // namespace dg
+
+extern "C" int dg_roe_flux_nodes(double gam, int form, int n, const double *qm, const double *qp, const double *nrm,
+                                 double *f2) {
+  if (n <= 0 || n > (1 << 26) || (form != 0 && form != 1) || !(gam > 1.0) || !qm || !qp || !nrm || !f2) {
+    g_bstate_err = "bad arguments";
+    return DG_ERR_ARG;
+  }
+  dg::Config c;
+  c.gam = gam;
+  const dg::Phys P = dg::make_phys(c);
+  const size_t m = (size_t)n;
+  double *d = nullptr;  // qm [n][4], qp [n][4], f2 [n][4], nrm [n][2]
+  cudaError_t ce = cudaMalloc(&d, m * 14 * sizeof(double));
+  if (ce == cudaSuccess) ce = cudaMemcpy(d, qm, m * 4 * sizeof(double), cudaMemcpyHostToDevice);
+  if (ce == cudaSuccess) ce = cudaMemcpy(d + 4 * m, qp, m * 4 * sizeof(double), cudaMemcpyHostToDevice);
+  if (ce == cudaSuccess) ce = cudaMemcpy(d + 12 * m, nrm, m * 2 * sizeof(double), cudaMemcpyHostToDevice);
+  if (ce == cudaSuccess) {
+    dg::roe_flux_kernel<<<(n + 127) / 128, 128>>>(n, form, d, d + 4 * m, d + 12 * m, P, d + 8 * m);
+    ce = cudaGetLastError();
+  }
+  if (ce == cudaSuccess) ce = cudaMemcpy(f2, d + 8 * m, m * 4 * sizeof(double), cudaMemcpyDeviceToHost);
+  if (d) cudaFree(d);
+  if (ce != cudaSuccess) {
+    g_bstate_err = std::string("dg_roe_flux_nodes: ") + cudaGetErrorString(ce);
+    return DG_ERR_CUDA;
+  }
+  return 0;
+}
+
 #include "dg_batch.cuh"
 #include "dg_adjoint.cuh"
 #include "dg_tangent.cuh"

@@ -347,6 +347,10 @@ int dg_tc_round(long long th, long long tl, int sc, double *out);
  * [n][4] receives twice the flux there, 0 elsewhere. */
 int dg_roe_pair_flux(double gam, int n, const double *qm, const double *qp, const double *nrm, int *taken,
                      double *f2);
+/* The same on the device: twice the Roe flux of n pairs of states as the face kernels compute it, form 0
+ * the general FP64 form, form 1 the rule (small-jump form where it applies).  Errors:
+ * dg_boundary_state_error(). */
+int dg_roe_flux_nodes(double gam, int form, int n, const double *qm, const double *qp, const double *nrm, double *f2);
 /* Cell ranges of the step graph for solvers whose graph is built from now on: 0 automatic (the
  * default: ranges of at least 128 tiles of 32 cells, at most 4), 1 a single range (the seven
  * launches as one chain), 2..32 that many ranges (fewer if the mesh has fewer tiles). */
