@@ -719,8 +719,8 @@ T *dptr(const op_arg &a) {
 
 // Device time of each loop: a pair of events around its launch, read later.  The loops run in stream
 // order without waiting for one another; only what hands a value to the host waits (calc_dt's and
-// l2_error's reductions, op_fetch_data), and there the finished pairs are read.  A wait after every
-// loop left the GPU idle for a launch and a host round trip 13 times a step.
+// l2_error's reductions, op_fetch_data, op_timers), and there (l2_error's apart) the finished pairs are read.  A wait after
+// every loop left the GPU idle for a launch and a host round trip 13 times a step.
 struct TimedPair {
   cudaEvent_t a, b;
   LoopStat *stat;
@@ -933,7 +933,9 @@ void op_fetch_data(op_dat dat, void *data) {
 
 int op_get_size(op_set set) { return set ? set->size : 0; }
 
+// The time when the loops called so far have finished, as after OP2's own loops, which wait each.
 void op_timers(double *cpu, double *wall) {
+  if (S().stream && ck(cudaStreamSynchronize(S().stream), "op_timers: an earlier loop")) read_timers();
   struct timeval t;
   gettimeofday(&t, nullptr);
   if (wall) *wall = t.tv_sec + t.tv_usec * 1e-6;

@@ -14,8 +14,13 @@
  *    copies it back.  Caller arrays are never written otherwise.
  *  - op_arg_gbl OP_READ values are read when the loop is called; OP_MAX
  *    results are written to the caller's variable before the loop returns.
- *  - each loop returns when its kernel has finished (as OP2's CUDA backend
- *    synchronises after every loop), so op_timing_output reports device times.
+ *  - loops run in the order they are called, on one stream; a loop returns when
+ *    its kernel has been launched.  What hands something to the host waits for
+ *    the loops before it: OP_MAX and OP_INC results, op_fetch_data, op2_gb300_sync and
+ *    op_timers, so that clocks read around loops cover their device time.
+ *    op_timing_output reports each loop's device time, read from events.
+ *  - an invalid call or launch fails in the loop itself; a fault while a kernel
+ *    runs is reported by the next call that waits or launches.
  *  - errors print a message and exit(1), as OP2 does
  *    (src/cuda/airfoil_kernels.cu:105); op2_gb300_set_exit_on_error(0) makes
  *    them return silently with the message in op2_gb300_last_error().
