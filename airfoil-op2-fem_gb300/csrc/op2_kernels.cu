@@ -805,6 +805,8 @@ void op2_gb300_reset(void) {
   State &s = S();
   if (s.stream) cudaStreamSynchronize(s.stream);
   read_timers();
+  for (cudaEvent_t e : TP().idle) cudaEventDestroy(e);
+  TP().idle.clear();
   for (auto &m : s.maps) cudaFree(m->d_data);
   for (auto &d : s.dats) cudaFree(d->d_data);
   for (auto &c : s.consts) cudaFree(c.second.second);
