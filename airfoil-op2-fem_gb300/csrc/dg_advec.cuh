@@ -369,12 +369,12 @@ __global__ void advec_vertex_kernel(int K, const int *cells, const int *owner, c
 
 // Element-kernel forms 2 and 3, and at every order but 3 form 1, run advec_fused_kernel; form 1 at
 // N = 3 the face kernel and the even/odd FP64 kernel, form 0 the face kernel and the dense one.
-static bool advec_fused(int N) { return g_elem_variant >= (N == 3 ? 2 : 1); }
+static bool advec_fused(int N) { return elem_form() >= (N == 3 ? 2 : 1); }
 
 template <int N>
 static void advec_launch_elem(const AdvInst &d, int stage, cudaStream_t s) {
   if constexpr (N == 3) {
-    if (g_elem_variant) {
+    if (elem_form()) {
       advec_elem_kernel_sym<N><<<(d.K + 31) / 32, 32 * np_of(N), 0, s>>>(d, stage);
       return;
     }
@@ -524,6 +524,8 @@ void Advection::enqueue_step_events(cudaStream_t s, cudaEvent_t *ev) {
 int Advection::step(int nsteps, bool use_graph, std::string &err) {
   auto capture = [&](int G, cudaGraph_t &g, cudaGraphExec_t &ex) -> int {
     if (ex) return 0;
+    if (!graph_exec && !graphG_exec) set = launch_set_now();  // for both graphs
+    const UseLaunchSet use(set);
     CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     for (int k = 0; k < G; k++) enqueue_step(stream);
     cudaError_t ce = cudaStreamEndCapture(stream, &g);

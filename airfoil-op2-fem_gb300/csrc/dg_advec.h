@@ -5,7 +5,7 @@
 #include <string>
 #include <vector>
 
-#include "dg_mesh.h"
+#include "dg_solver.h"
 
 namespace dg {
 
@@ -33,6 +33,7 @@ struct Advection {
   static constexpr int kGraphSteps = 8;  // steps of the longer graph that runs launch where it fits
   cudaGraph_t graphG = nullptr;
   cudaGraphExec_t graphG_exec = nullptr;
+  LaunchSet set;  // the launch settings of both
   double *coords_d = nullptr;
   int *cells_d = nullptr;
   std::vector<void *> allocs;

@@ -170,9 +170,9 @@ static BatchVariant batch_variant() {
 // The persistent kernels of the current element-kernel form (the batch computes exactly what the
 // plain solvers compute).
 static std::vector<BatchVariant> batch_variants() {
-  if (g_elem_variant == 3)
+  if (elem_form() == 3)
     return {batch_variant<512, 1, 2>(), batch_variant<512, 2, 2>(), batch_variant<1024, 1, 2>()};
-  if (g_elem_variant == 2)
+  if (elem_form() == 2)
     return {batch_variant<512, 1, 1>(), batch_variant<512, 2, 1>(), batch_variant<1024, 1, 1>()};
   return {batch_variant<512, 1, 0>(), batch_variant<512, 2, 0>(), batch_variant<1024, 1, 0>()};
 }
@@ -276,7 +276,7 @@ struct Batch {
   // chooses them for a mesh of all the order's cells), higher orders first; face tiles of ft nodes.
   int build_tiles(int ft, bool grouped, std::string &err) {
     std::vector<int4> et, fts;
-    form = g_elem_variant;
+    form = elem_form();
     for (int n = 6; n >= 1; n--) {
       ord_first[n] = (int)et.size();
       ord_small[n] = grouped && (form == 3 || n == 6) &&
@@ -398,10 +398,10 @@ struct Batch {
         DG_DISPATCH(n, (batch_elem_small_kernel<NN>
                         <<<ord_count[n], elem_small_threads(NN), elem_sym_smem(NN, elem_small_ct(NN)), s>>>(
                             d_insts, d_etiles, ord_first[n], stage)));
-      } else if (g_elem_variant == 3) {
+      } else if (elem_form() == 3) {
         DG_DISPATCH(n, (batch_elem_kernel<NN, 2><<<ord_count[n], 32 * np_of(NN), sm, s>>>(d_insts, d_etiles,
                                                                                           ord_first[n], stage)));
-      } else if (g_elem_variant == 2) {
+      } else if (elem_form() == 2) {
         DG_DISPATCH(n, (batch_elem_kernel<NN, 1><<<ord_count[n], 32 * np_of(NN), sm, s>>>(d_insts, d_etiles,
                                                                                           ord_first[n], stage)));
       } else {
@@ -570,7 +570,7 @@ struct Batch {
 
   int run(int nsteps, std::string &err) {
     if (int rc = ensure_shape(err)) return rc;
-    if (!graph_exec && form != g_elem_variant)  // the tiles follow the form until a graph holds them
+    if (!graph_exec && form != elem_form())  // the tiles follow the form until a graph holds them
       if (int rc = set_shape(shape.variant, shape.face_tile, shape, err)) return rc;
     if (!graph_exec && graph_ok) {
       std::string gerr;
@@ -581,7 +581,7 @@ struct Batch {
       // several steps per graph launch, as the plain solver (see g_steps_per_graph)
       std::string gerr;
       if (!graphG_exec) graph_steps = steps_per_graph();
-      if (graph_steps > 1 && nsteps >= graph_steps && !graphG_exec && form == g_elem_variant)
+      if (graph_steps > 1 && nsteps >= graph_steps && !graphG_exec && form == elem_form())
         capture_steps(graph_steps, graphG, graphG_exec, gerr);
       if (graphG_exec)
         for (; i + graph_steps <= nsteps; i += graph_steps) {

@@ -968,7 +968,15 @@ static std::atomic<int> g_pdl{1};
 // Set by this thread while it enqueues the step graph over cell ranges without programmatic
 // launch (the process-wide setting stays as it is for other threads).
 static thread_local int t_no_pdl = 0;
-static inline bool pdl_on() { return g_pdl.load(std::memory_order_relaxed) && !t_no_pdl; }
+// The settings under which this thread enqueues launches while it captures a solver's graph, null
+// otherwise (then the process-wide ones).
+static thread_local const LaunchSet *t_set = nullptr;
+static LaunchSet launch_set_now();
+struct UseLaunchSet {
+  explicit UseLaunchSet(const LaunchSet &ls) { t_set = &ls; }
+  ~UseLaunchSet() { t_set = nullptr; }
+};
+static inline bool pdl_on() { return (t_set ? t_set->pdl : g_pdl.load(std::memory_order_relaxed)) && !t_no_pdl; }
 
 // Scheduling priority given to the launches this thread makes while g_launch_prio_on is set (the
 // step graph over cell ranges sets it per range; lower numbers are scheduled first).
@@ -1002,8 +1010,8 @@ static void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
 template <int N>
 static void launch_face(const Inst &d, int stage, cudaStream_t s) {
   const long long nf = ((long long)d.nE + d.nB) * (N + 1);
-  const int bs = g_face_block;
-  if (g_face_r64 && bs == 64)
+  const int bs = t_set ? t_set->face_block : (int)g_face_block;
+  if ((t_set ? t_set->face_r64 : (int)g_face_r64) && bs == 64)
     launch_pdl(face_kernel_r64<N>, dim3((unsigned)((nf + bs - 1) / bs)), dim3(bs), 0, s, d, stage);
   else
     launch_pdl(face_kernel<N>, dim3((unsigned)((nf + bs - 1) / bs)), dim3(bs), 0, s, d, stage);
@@ -1014,6 +1022,7 @@ static void launch_face(const Inst &d, int stage, cudaStream_t s) {
 // 2: even/odd with the contraction on the tensor cores (from N = 3 on, in FP64 at N = 1, 2),
 // 1: even/odd in FP64 (on the tensor cores at N = 6), 0: dense FP64.
 static std::atomic<int> g_elem_variant{3};
+static inline int elem_form() { return t_set ? t_set->form : (int)g_elem_variant; }
 
 // The even/odd element kernel instance for form TC at order N, launched over tiles [t0, t1):
 // with the launch attributes of launch_pdl (attr true) or as a plain launch.  The instance
@@ -1038,11 +1047,13 @@ static void elem_sym_launch(const Inst &d, int stage, int t0, int t1, cudaStream
 // 61 / 57 / 74 us against 46 / 51 / 61 us): its 8 contraction warps per SM run the integer-heavy
 // product with too little parallelism, where the one-tile blocks bring 30 warps per SM to it.
 static std::atomic<int> g_elem_ws{0};
+static inline int elem_ws_mode() { return t_set ? t_set->ws : (int)g_elem_ws; }
 
 // Resident blocks per SM that the order-3 tensor-core element kernel is compiled for: 3 (the
 // default: 64 registers, a small spill) or 2 (more registers, no spill, and room beside two
 // element blocks for face-kernel blocks of another cell range in the step graph).
 static std::atomic<int> g_elem_mb{3};
+static inline int elem_mb() { return t_set ? t_set->mb : (int)g_elem_mb; }
 
 static int ws_sm_count() {
   static int sms[kMaxDevices] = {0};
@@ -1055,7 +1066,7 @@ static int ws_sm_count() {
 template <int N>
 static void elem_ws_launch(const Inst &d, int stage, int t0, int t1, cudaStream_t s, bool attr) {
   const int T = (d.K + 31) / 32, sms = ws_sm_count();
-  int grid = g_elem_ws == 2 ? (int)(((long long)sms * (t1 - t0) + T - 1) / T) : sms;
+  int grid = elem_ws_mode() == 2 ? (int)(((long long)sms * (t1 - t0) + T - 1) / T) : sms;
   grid = std::max(1, std::min(grid, t1 - t0));
   const size_t smem = ws_smem(N);
   if (attr && pdl_on())
@@ -1110,21 +1121,21 @@ template <int N>
 static void launch_elem_form(const Inst &d, int stage, int t0, int t1, cudaStream_t s, bool attr) {
   if (t1 <= t0) return;
   if constexpr (elem_small_used(N)) {
-    if ((g_elem_variant == 3 || N == 6) && !(g_elem_ws && ws_used(N)) && elem_small(N, d.K))
+    if ((elem_form() == 3 || N == 6) && !(elem_ws_mode() && ws_used(N)) && elem_small(N, d.K))
       return elem_small_launch<N>(d, stage, 32 * t0, 32 * t1, s, attr);
   }
   if constexpr (ws_used(N)) {
-    if (g_elem_ws && g_elem_variant >= 2) return elem_ws_launch<N>(d, stage, t0, t1, s, attr);
+    if (elem_ws_mode() && elem_form() >= 2) return elem_ws_launch<N>(d, stage, t0, t1, s, attr);
   }
   if constexpr (ozd_used(N, 2)) {
-    if (g_elem_variant == 3) return elem_sym_launch<N, 2, oz_min_blocks(N)>(d, stage, t0, t1, s, attr);
+    if (elem_form() == 3) return elem_sym_launch<N, 2, oz_min_blocks(N)>(d, stage, t0, t1, s, attr);
   }
   if constexpr (oz_used(N, 1)) {
     if constexpr (N == 3) {
       // the register budget of two resident blocks per SM instead of three (g_elem_mb)
-      if (g_elem_variant >= 2 && g_elem_mb == 2) return elem_sym_launch<N, 1, 2>(d, stage, t0, t1, s, attr);
+      if (elem_form() >= 2 && elem_mb() == 2) return elem_sym_launch<N, 1, 2>(d, stage, t0, t1, s, attr);
     }
-    if (g_elem_variant >= 2) return elem_sym_launch<N, 1, oz_min_blocks(N)>(d, stage, t0, t1, s, attr);
+    if (elem_form() >= 2) return elem_sym_launch<N, 1, oz_min_blocks(N)>(d, stage, t0, t1, s, attr);
   }
   elem_sym_launch<N, 0, 1>(d, stage, t0, t1, s, attr);
 }
@@ -1132,7 +1143,7 @@ static void launch_elem_form(const Inst &d, int stage, int t0, int t1, cudaStrea
 template <int N>
 static void launch_elem(const Inst &d, int stage, cudaStream_t s) {
   constexpr int Np = np_of(N), NK = nk_of(N);
-  if (g_elem_variant) {
+  if (elem_form()) {
     launch_elem_form<N>(d, stage, 0, (d.K + 31) / 32, s, true);
   } else {
     const size_t smem = (size_t)NK * 32 * 4 * sizeof(double);
@@ -1592,11 +1603,12 @@ void Solver::enqueue_step_events(cudaStream_t s, cudaEvent_t *ev) {
   cudaEventRecord(ev[7], s);
 }
 
-// The cell ranges of this solver's step graphs and the steps in one of them (once, and again after
-// drop_graphs).
+// The launch settings and cell ranges of this solver's step graphs and the steps in one of them (once,
+// and again after drop_graphs).
 int Solver::build_graph(std::string &err) {
   if (parts) return 0;
-  const int P = g_elem_variant ? step_parts_for(K) : 1;  // the dense FP64 form has no tile ranges
+  set = launch_set_now();
+  const int P = set.form ? step_parts_for(K) : 1;  // the dense FP64 form has no tile ranges
   if (P > 1) {
     if (int rc = build_parts(P, err)) return rc;
   } else {
@@ -1609,7 +1621,8 @@ int Solver::build_graph(std::string &err) {
 // G steps as one graph; captured when a run first needs it.
 int Solver::capture_steps(int G, cudaGraph_t &gr, cudaGraphExec_t &ex, std::string &err) {
   if (ex) return 0;
-  const unsigned long long flags = (parts > 1 && (step_graph_flags() & 6)) ? cudaGraphInstantiateFlagUseNodePriority : 0;
+  const UseLaunchSet use(set);
+  const unsigned long long flags = (parts > 1 && (set.graph_flags & 6)) ? cudaGraphInstantiateFlagUseNodePriority : 0;
   CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
   if (parts > 1) enqueue_step_parts(stream, nullptr, nullptr, G);
   else
@@ -1641,6 +1654,17 @@ static std::atomic<int> g_step_parts{0};  // 0: automatic (step_parts_for), 1: t
 // could use: 300 vs 267 us per step at 4 ranges); bit 1: give range p's launches a scheduling
 // priority that falls with p (earlier ranges first; measured no faster).
 static std::atomic<int> g_step_graph_flags{1};
+static LaunchSet launch_set_now() {
+  LaunchSet ls;
+  ls.form = g_elem_variant;
+  ls.ws = g_elem_ws;
+  ls.mb = g_elem_mb;
+  ls.pdl = g_pdl;
+  ls.face_block = g_face_block;
+  ls.face_r64 = g_face_r64;
+  ls.graph_flags = g_step_graph_flags;
+  return ls;
+}
 void set_step_graph_flags(int f) { g_step_graph_flags = f & 7; }
 int step_graph_flags() { return g_step_graph_flags; }
 
@@ -1748,15 +1772,16 @@ void Solver::enqueue_step_parts(cudaStream_t s, const double *q_in, double *q_ou
     c0 = (size_t)ptile0[p] * 32;
     nc = std::min((size_t)ptile0[p + 1] * 32, (size_t)K) - c0;
   };
-  t_no_pdl = (g_step_graph_flags & 1) ? 1 : 0;
+  const int gflags = set.graph_flags;
+  t_no_pdl = (gflags & 1) ? 1 : 0;
   int prio_lo = 0, prio_hi = 0;  // least and greatest priority (numerically: hi <= lo)
   cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
   // bit 1: earlier ranges first; bit 2: element launches before face launches
   auto set_prio = [&](int p, bool elem) {
-    if (g_step_graph_flags & 2) {
+    if (gflags & 2) {
       g_launch_prio_on = 1;
       g_launch_prio = prio_hi + (int)((long long)(prio_lo - prio_hi) * p / std::max(1, P - 1));
-    } else if (g_step_graph_flags & 4) {
+    } else if (gflags & 4) {
       g_launch_prio_on = 1;
       g_launch_prio = elem ? prio_hi : prio_lo;
     }
@@ -1850,6 +1875,7 @@ int Solver::step_io_parts(const double *q_in, double *q_out, bool &done, std::st
   if (!io_graph_exec || io_in != q_in || io_out != q_out) {
     if (io_graph_exec) { cudaGraphExecDestroy(io_graph_exec); io_graph_exec = nullptr; }
     if (io_graph) { cudaGraphDestroy(io_graph); io_graph = nullptr; }
+    const UseLaunchSet use(set);
     CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     enqueue_step_parts(stream, q_in, q_out);
     cudaError_t ce = cudaStreamEndCapture(stream, &io_graph);

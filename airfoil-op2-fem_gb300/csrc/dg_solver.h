@@ -19,6 +19,15 @@ struct Config {
   double vortex_x0 = 5.0, vortex_y0 = 0.0, vortex_beta = 5.0;
 };
 
+// The launch settings of the plain path and the advection app (dg_set_elem_variant, dg_set_elem_ws,
+// dg_set_elem_blocks_per_sm, dg_set_pdl, dg_set_face_block, dg_set_face_regs64, dg_set_step_graph_flags)
+// as one value.  A solver's step graphs (one step, several, with host copies) are captured when a call
+// first needs each; all of them are captured under the settings that the first one found, so that
+// every step of a solver has the same arithmetic.
+struct LaunchSet {
+  int form = 3, ws = 0, mb = 3, pdl = 1, face_block = 64, face_r64 = 0, graph_flags = 1;
+};
+
 // Device step state of one instance.
 struct StepState {
   double dt;                    // current time step
@@ -131,7 +140,8 @@ struct Solver {
   int capture_steps(int G, cudaGraph_t &gr, cudaGraphExec_t &ex, std::string &err);
   // The step graph as a DAG of cell ranges (build_graph with more than one range).
   std::vector<int4> h_edges, h_bedges;  // device edge records in mesh order (host copy)
-  int parts = 0;                         // ranges of the graph built (0: none yet)
+  int parts = 0;                         // ranges of the graphs built (0: none yet)
+  LaunchSet set;                         // their launch settings
   int4 *pedges = nullptr, *pbedges = nullptr;  // edge records sorted by range
   double *pbxy = nullptr;                // boundary node coordinates in that order
   std::vector<int> ptile0, pe0, pb0, plo, phi;

@@ -308,7 +308,8 @@ double dg_fp64_mma_peak_gflops(void);
 double dg_f16_mma_peak_gflops(void);
 /* Number of kernels one dg_solver_run step launches. */
 int dg_kernels_per_step(void);
-/* Element-kernel form for launches and graphs built from now on: 3 (default) the dense rows
+/* Element-kernel form for launches from now on (a solver's step graphs keep the form, and the other
+ * settings below, that its first run found): 3 (default) the dense rows
  * [Drw | Dsw | -LIFT] on the tensor cores as an exact integer product at orders N = 1, 2 and
  * the even/odd split there at the other orders; 2 the even/odd split of those rows with its contraction on the
  * tensor cores from N = 3 on and in FP64 at N = 1, 2; 1 the even/odd split in FP64 (at N = 6 on the
