@@ -323,20 +323,18 @@ struct Batch {
       for (int n = 1; n <= 6; n++) {
         const size_t sm = elem_sym_smem(n);
         cudaError_t ce = cudaSuccess;
-        DG_DISPATCH(n, ce = cudaFuncSetAttribute(batch_elem_kernel<NN, 0>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        if (ce == cudaSuccess) {
-          DG_DISPATCH(n, ce = cudaFuncSetAttribute(batch_elem_kernel<NN, 1>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        }
-        if (ce == cudaSuccess) {
-          DG_DISPATCH(n, ce = cudaFuncSetAttribute(batch_elem_kernel<NN, 2>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        }
-        if (ce == cudaSuccess) {
-          DG_DISPATCH(n, ce = cudaFuncSetAttribute(batch_elem_small_kernel<NN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)elem_sym_smem(NN, elem_small_ct(NN))));
-        }
+        auto limit = [&](auto kernel, size_t bytes) {
+          if (ce == cudaSuccess)
+            ce = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        };
+        DG_DISPATCH(n, {
+          if constexpr (NN != 6) {
+            limit(batch_elem_kernel<NN, 0>, sm);
+            limit(batch_elem_kernel<NN, 1>, sm);
+          }
+          if constexpr (!elem_small_only(NN)) limit(batch_elem_kernel<NN, 2>, sm);
+          limit(batch_elem_small_kernel<NN>, elem_sym_smem(NN, elem_small_ct(NN)));
+        });
         if (ce != cudaSuccess) { err = cudaGetErrorString(ce); return -100; }
       }
       if (int rc = build_tiles(ft, true, err)) return rc;
@@ -394,20 +392,18 @@ struct Batch {
     for (int n = 6; n >= 1; n--) {
       if (!ord_count[n]) continue;
       const size_t sm = elem_sym_smem(n);
-      if (ord_small[n]) {
-        DG_DISPATCH(n, (batch_elem_small_kernel<NN>
-                        <<<ord_count[n], elem_small_threads(NN), elem_sym_smem(NN, elem_small_ct(NN)), s>>>(
-                            d_insts, d_etiles, ord_first[n], stage)));
-      } else if (elem_form() == 3) {
-        DG_DISPATCH(n, (batch_elem_kernel<NN, 2><<<ord_count[n], 32 * np_of(NN), sm, s>>>(d_insts, d_etiles,
-                                                                                          ord_first[n], stage)));
-      } else if (elem_form() == 2) {
-        DG_DISPATCH(n, (batch_elem_kernel<NN, 1><<<ord_count[n], 32 * np_of(NN), sm, s>>>(d_insts, d_etiles,
-                                                                                          ord_first[n], stage)));
-      } else {
-        DG_DISPATCH(n, (batch_elem_kernel<NN, 0><<<ord_count[n], 32 * np_of(NN), sm, s>>>(d_insts, d_etiles,
-                                                                                          ord_first[n], stage)));
-      }
+      const int f = ord_first[n];
+      DG_DISPATCH(n, {
+        const dim3 g(ord_count[n]), b(32 * np_of(NN));
+        if (ord_small[n]) {
+          batch_elem_small_kernel<NN><<<g, elem_small_threads(NN), elem_sym_smem(NN, elem_small_ct(NN)), s>>>(
+              d_insts, d_etiles, f, stage);
+        } else if constexpr (NN != 6) {
+          if (form == 2) batch_elem_kernel<NN, 1><<<g, b, sm, s>>>(d_insts, d_etiles, f, stage);
+          else if (form != 3) batch_elem_kernel<NN, 0><<<g, b, sm, s>>>(d_insts, d_etiles, f, stage);
+          else if constexpr (!elem_small_only(NN)) batch_elem_kernel<NN, 2><<<g, b, sm, s>>>(d_insts, d_etiles, f, stage);
+        }
+      });
     }
     return cudaGetLastError();
   }

@@ -425,7 +425,7 @@ constexpr int kElemSlot = elem_slot(32);
 // Small tiles: the orders whose contraction is on the tensor cores, their cells, the threads of a
 // block (one per cell and node, and at least a warp per unit of the contraction) and, of a tile of
 // CT cells, the threads per column of the operand pre-pass.
-constexpr bool elem_small_used(int N) { return N >= 1 && N <= kOzMaxN; }
+constexpr bool elem_small_only(int N) { return N == 2 || N == 6; }  // form 3 has no 32-cell tiles (elem_small)
 constexpr int elem_small_ct(int N) { return N == 2 ? 16 : 8; }
 constexpr int elem_small_units(int N) { return N <= 2 ? 1 : (N == 3 ? 2 : (N == 4 ? 3 : 4)); }  // n-tiles
 constexpr int elem_small_threads(int N) {

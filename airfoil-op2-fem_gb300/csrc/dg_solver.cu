@@ -1120,24 +1120,26 @@ static void elem_small_launch(const Inst &d, int stage, int c0, int c1, cudaStre
 template <int N>
 static void launch_elem_form(const Inst &d, int stage, int t0, int t1, cudaStream_t s, bool attr) {
   if (t1 <= t0) return;
-  if constexpr (elem_small_used(N)) {
-    if ((elem_form() == 3 || N == 6) && !(elem_ws_mode() && ws_used(N)) && elem_small(N, d.K))
+  if constexpr (N == 6) {  // forms 1 to 3 alike
+    elem_small_launch<N>(d, stage, 32 * t0, 32 * t1, s, attr);
+  } else {
+    if (elem_form() == 3 && !(elem_ws_mode() && ws_used(N)) && elem_small(N, d.K))
       return elem_small_launch<N>(d, stage, 32 * t0, 32 * t1, s, attr);
-  }
-  if constexpr (ws_used(N)) {
-    if (elem_ws_mode() && elem_form() >= 2) return elem_ws_launch<N>(d, stage, t0, t1, s, attr);
-  }
-  if constexpr (ozd_used(N, 2)) {
-    if (elem_form() == 3) return elem_sym_launch<N, 2, oz_min_blocks(N)>(d, stage, t0, t1, s, attr);
-  }
-  if constexpr (oz_used(N, 1)) {
-    if constexpr (N == 3) {
-      // the register budget of two resident blocks per SM instead of three (g_elem_mb)
-      if (elem_form() >= 2 && elem_mb() == 2) return elem_sym_launch<N, 1, 2>(d, stage, t0, t1, s, attr);
+    if constexpr (ws_used(N)) {
+      if (elem_ws_mode() && elem_form() >= 2) return elem_ws_launch<N>(d, stage, t0, t1, s, attr);
     }
-    if (elem_form() >= 2) return elem_sym_launch<N, 1, oz_min_blocks(N)>(d, stage, t0, t1, s, attr);
+    if constexpr (ozd_used(N, 2) && !elem_small_only(N)) {
+      if (elem_form() == 3) return elem_sym_launch<N, 2, oz_min_blocks(N)>(d, stage, t0, t1, s, attr);
+    }
+    if constexpr (oz_used(N, 1)) {
+      if constexpr (N == 3) {
+        // the register budget of two resident blocks per SM instead of three (g_elem_mb)
+        if (elem_form() >= 2 && elem_mb() == 2) return elem_sym_launch<N, 1, 2>(d, stage, t0, t1, s, attr);
+      }
+      if (elem_form() >= 2) return elem_sym_launch<N, 1, oz_min_blocks(N)>(d, stage, t0, t1, s, attr);
+    }
+    elem_sym_launch<N, 0, 1>(d, stage, t0, t1, s, attr);
   }
-  elem_sym_launch<N, 0, 1>(d, stage, t0, t1, s, attr);
 }
 
 template <int N>
@@ -1179,18 +1181,15 @@ static cudaError_t set_smem_attr() {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pdl, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_sym);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_plain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_sym);
   };
-  both(elem_kernel_sym<N, 0, 1, true>, elem_kernel_sym<N, 0, 1, false>);
-  if constexpr (oz_used(N, 1))
+  if constexpr (N != 6) both(elem_kernel_sym<N, 0, 1, true>, elem_kernel_sym<N, 0, 1, false>);
+  if constexpr (oz_used(N, 1) && N != 6)
     both(elem_kernel_sym<N, 1, oz_min_blocks(N), true>, elem_kernel_sym<N, 1, oz_min_blocks(N), false>);
   if constexpr (N == 3) both(elem_kernel_sym<N, 1, 2, true>, elem_kernel_sym<N, 1, 2, false>);
-  if constexpr (ozd_used(N, 2))
+  if constexpr (ozd_used(N, 2) && !elem_small_only(N))
     both(elem_kernel_sym<N, 2, oz_min_blocks(N), true>, elem_kernel_sym<N, 2, oz_min_blocks(N), false>);
-  if constexpr (elem_small_used(N)) {
-    for (auto k : {elem_kernel_small<N, true>, elem_kernel_small<N, false>})
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)elem_sym_smem(N, elem_small_ct(N)));
-  }
+  for (auto k : {elem_kernel_small<N, true>, elem_kernel_small<N, false>})
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)elem_sym_smem(N, elem_small_ct(N)));
   if constexpr (ws_used(N)) {
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(elem_kernel_ws<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ws_smem(N));

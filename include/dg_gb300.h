@@ -313,7 +313,8 @@ int dg_kernels_per_step(void);
  * [Drw | Dsw | -LIFT] on the tensor cores as an exact integer product at orders N = 1, 2 and
  * the even/odd split there at the other orders; 2 the even/odd split of those rows with its contraction on the
  * tensor cores from N = 3 on and in FP64 at N = 1, 2; 1 the even/odd split in FP64 (at N = 6 on the
- * tensor cores, as in forms 2 and 3); 0 dense FP64 rows.  All compute the same right-hand side to rounding (the tensor-core
+ * tensor cores, as in forms 2 and 3); 0 dense FP64 rows.  The advection app has the dense FP64 rows in
+ * form 0, the even/odd split in FP64 in form 1 at N = 3, and the tensor cores otherwise.  All compute the same right-hand side to rounding (the tensor-core
  * contraction is the correctly rounded dot product of the 56-bit truncated inputs). */
 void dg_set_elem_variant(int variant);
 /* The current element-kernel form. */
