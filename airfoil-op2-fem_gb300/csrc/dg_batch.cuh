@@ -280,7 +280,7 @@ struct Batch {
     for (int n = 6; n >= 1; n--) {
       ord_first[n] = (int)et.size();
       ord_small[n] = grouped && (form == 3 || n == 6) &&
-                     elem_small(n, (int)std::min<long long>(ord_cells[n], 0x7FFFFFFF));
+                     elem_small(n, (int)std::min<long long>(ord_cells[n], 0x7FFFFFFF), sm_count_now());
       const int ct = ord_small[n] ? elem_small_ct(n) : 32;
       for (size_t k = 0; k < solvers.size(); k++) {
         if (cfgs[k].N != n) continue;

@@ -1055,7 +1055,8 @@ static inline int elem_ws_mode() { return t_set ? t_set->ws : (int)g_elem_ws; }
 static std::atomic<int> g_elem_mb{3};
 static inline int elem_mb() { return t_set ? t_set->mb : (int)g_elem_mb; }
 
-static int ws_sm_count() {
+// SMs of the current device.
+static int sm_count_now() {
   static int sms[kMaxDevices] = {0};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 1;
@@ -1065,7 +1066,7 @@ static int ws_sm_count() {
 
 template <int N>
 static void elem_ws_launch(const Inst &d, int stage, int t0, int t1, cudaStream_t s, bool attr) {
-  const int T = (d.K + 31) / 32, sms = ws_sm_count();
+  const int T = (d.K + 31) / 32, sms = sm_count_now();
   int grid = elem_ws_mode() == 2 ? (int)(((long long)sms * (t1 - t0) + T - 1) / T) : sms;
   grid = std::max(1, std::min(grid, t1 - t0));
   const size_t smem = ws_smem(N);
@@ -1087,20 +1088,26 @@ static void elem_ws_launch(const Inst &d, int stage, int t0, int t1, cudaStream_
 //   N = 2: 2048 57.4 / 55.9, 32768 131.0 / 115.4, 262144 896 / 788 us
 //   N = 3: 2048 70.9 / 55.7, 8192 85.7 / 77.7, 14000 111.9 / 103.6, 28000 162.9 / 163.9 us
 //   N = 4: 1152 86.2 / 63.8, 8192 114.2 / 112.7, 9600 115.9 / 118.8, 28000 255.7 / 275.9 us
-//   N = 5: 1152 74.9 / 64.6, 3072 88.1 / 96.9, 6000 157.8 / 138.1, 9600 165.9 / 179.2,
-//          28000 423.7 / 410.3, 262144 3784 / 3714 us
-// (N = 5 keeps 32 cells where their blocks, one per SM, nearly fill one or two waves; N = 6, whose
-// 32-cell block would hold 896 threads and 109 KB, has the small tiles only).
-static bool elem_small(int N, int K) {
+//   N = 5: 1152 74.9 / 64.6, 3072 88.1 / 96.9, 6400 153.1 / 138.6, 7680 161.2 / 153.4, 8192 161.4 /
+//          160.7, 9600 165.9 / 179.2, 28000 423.7 / 410.3, 262144 3784 / 3714 us
+// At N = 5 a 32-cell block has an SM to itself: it keeps 32 cells where T such tiles fill more than half
+// of one wave over the SMs (3072 cells: 0.63 waves) or more than 11/16 of the second (8192 cells, 1.68
+// waves, is where the two meet).  N = 6, whose 32-cell block would hold 896 threads and 109 KB, has the
+// small tiles only.  sms: SMs of the device (152 above).
+static constexpr bool elem_small(int N, int K, int sms) {
+  const long long T = ((long long)K + 31) / 32;
   switch (N) {
     case 1: return K <= 32768;
     case 2: return true;
     case 3: return K <= 20480;
     case 4: return K <= 8192;
-    case 5: return !((K > 16 * 152 && K <= 32 * 152) || (K > 8192 && K <= 64 * 152));
+    case 5: return !((2 * T > sms && T <= sms) || (16 * T > 27 * (long long)sms && T <= 2 * (long long)sms));
     default: return true;
   }
 }
+static_assert(elem_small(5, 2432, 152) && !elem_small(5, 2433, 152) && !elem_small(5, 4864, 152) && elem_small(5, 4865, 152));
+static_assert(elem_small(5, 8192, 152) && !elem_small(5, 8193, 152) && !elem_small(5, 9728, 152) && elem_small(5, 9729, 152));
+static_assert(!elem_small(5, 32 * 100, 100) && elem_small(5, 32 * 101, 100) && !elem_small(5, 32 * 200, 100));
 
 template <int N>
 static void elem_small_launch(const Inst &d, int stage, int c0, int c1, cudaStream_t s, bool attr) {
@@ -1123,7 +1130,7 @@ static void launch_elem_form(const Inst &d, int stage, int t0, int t1, cudaStrea
   if constexpr (N == 6) {  // forms 1 to 3 alike
     elem_small_launch<N>(d, stage, 32 * t0, 32 * t1, s, attr);
   } else {
-    if (elem_form() == 3 && !(elem_ws_mode() && ws_used(N)) && elem_small(N, d.K))
+    if (elem_form() == 3 && !(elem_ws_mode() && ws_used(N)) && elem_small(N, d.K, N == 5 ? sm_count_now() : 0))
       return elem_small_launch<N>(d, stage, 32 * t0, 32 * t1, s, attr);
     if constexpr (ws_used(N)) {
       if (elem_ws_mode() && elem_form() >= 2) return elem_ws_launch<N>(d, stage, t0, t1, s, attr);
