@@ -274,37 +274,51 @@ struct Batch {
 
   // Element tiles (32 cells of one instance; with grouped launches small tiles where elem_small
   // chooses them for a mesh of all the order's cells), higher orders first; face tiles of ft nodes.
+  // The graphs hold the old tiles and go with them; on failure both stay as they were.
   int build_tiles(int ft, bool grouped, std::string &err) {
     std::vector<int4> et, fts;
-    form = elem_form();
+    const int fm = elem_form();
+    int first[7] = {0}, count[7] = {0};
+    bool small[7] = {false};
     for (int n = 6; n >= 1; n--) {
-      ord_first[n] = (int)et.size();
-      ord_small[n] = grouped && (form == 3 || n == 6) &&
-                     elem_small(n, (int)std::min<long long>(ord_cells[n], 0x7FFFFFFF), sm_count_now());
-      const int ct = ord_small[n] ? elem_small_ct(n) : 32;
+      first[n] = (int)et.size();
+      small[n] = grouped && (fm == 3 || n == 6) &&
+                 elem_small(n, (int)std::min<long long>(ord_cells[n], 0x7FFFFFFF), sm_count_now());
+      const int ct = small[n] ? elem_small_ct(n) : 32;
       for (size_t k = 0; k < solvers.size(); k++) {
         if (cfgs[k].N != n) continue;
         const int K = solvers[k]->K;
         for (int e0 = 0; e0 < K; e0 += ct) et.push_back(make_int4((int)k, e0, 0, n));
       }
-      ord_count[n] = (int)et.size() - ord_first[n];
+      count[n] = (int)et.size() - first[n];
     }
     for (size_t k = 0; k < solvers.size(); k++) {
       const Inst &d = solvers[k]->d;
       const int total = (d.nE + d.nB) * (d.N + 1);
       for (int f0 = 0; f0 < total; f0 += ft) fts.push_back(make_int4((int)k, f0, std::min(ft, total - f0), d.N));
     }
-    if (d_ftiles) cudaFree(d_ftiles);
-    if (d_etiles) cudaFree(d_etiles);
-    d_ftiles = d_etiles = nullptr;
-    if (cudaMalloc(&d_ftiles, sizeof(int4) * fts.size()) != cudaSuccess ||
-        cudaMalloc(&d_etiles, sizeof(int4) * et.size()) != cudaSuccess) {
-      err = "cudaMalloc failed";
+    int4 *df = nullptr, *de = nullptr;
+    cudaError_t ce = cudaMalloc(&df, sizeof(int4) * fts.size());
+    if (ce == cudaSuccess) ce = cudaMalloc(&de, sizeof(int4) * et.size());
+    if (ce == cudaSuccess) ce = cudaMemcpy(df, fts.data(), sizeof(int4) * fts.size(), cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) ce = cudaMemcpy(de, et.data(), sizeof(int4) * et.size(), cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(stream);  // steps in flight read the old tiles
+    if (ce != cudaSuccess) {
+      cudaGetLastError();
+      if (df) cudaFree(df);
+      if (de) cudaFree(de);
+      err = cudaGetErrorString(ce);
       return -100;
     }
-    cudaError_t ce = cudaMemcpy(d_ftiles, fts.data(), sizeof(int4) * fts.size(), cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess) ce = cudaMemcpy(d_etiles, et.data(), sizeof(int4) * et.size(), cudaMemcpyHostToDevice);
-    if (ce != cudaSuccess) { err = cudaGetErrorString(ce); return -100; }
+    drop_graphs();
+    if (d_ftiles) cudaFree(d_ftiles);
+    if (d_etiles) cudaFree(d_etiles);
+    d_ftiles = df;
+    d_etiles = de;
+    form = fm;
+    std::copy(first, first + 7, ord_first);
+    std::copy(count, count + 7, ord_count);
+    std::copy(small, small + 7, ord_small);
     nft = (int)fts.size();
     net = (int)et.size();
     return 0;
@@ -471,10 +485,13 @@ struct Batch {
       if (ce == cudaSuccess) ce = cudaMemcpy(s->d.st, &s0[k], sizeof(StepState), cudaMemcpyHostToDevice);
       if (ce != cudaSuccess) { err = cudaGetErrorString(ce); return -100; }
     }
-    if (best.variant < 0) { err = "no batched launch shape ran"; return -7; }
+    if (best.variant < 0) {  // the tiles are the last candidate's: the next run makes its own
+      shape = BatchShape();
+      err = "no batched launch shape ran";
+      return -7;
+    }
     if (int rc = set_shape(best.variant, best.face_tile, shape, err)) return rc;
     shape.ms_per_step = best.ms_per_step;
-    drop_graphs();
     return 0;
   }
 

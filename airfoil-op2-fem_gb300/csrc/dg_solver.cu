@@ -2435,7 +2435,6 @@ extern "C" int dg_batch_use_shape(dg_batch_t *h, int variant, int face_tile) {
   dg::BatchShape sh;
   if (h->b.set_shape(variant, face_tile, sh, err)) return batch_fail(DG_ERR_ARG, err);
   h->b.shape = sh;
-  h->b.drop_graphs();
   h->b.graph_ok = true;
   return 0;
 }
