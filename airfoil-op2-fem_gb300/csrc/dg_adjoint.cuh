@@ -29,7 +29,7 @@
 // also keeps the last segment's stages in the segment buffers the reverse sweep starts with; going
 // backwards, each earlier segment is re-run from its checkpoint with the frozen dt sequence,
 // keeping q, W1, W2 of each of its steps.  (K = 32768, N = 3, 40 steps in two segments, forward and
-// backward: 39.8 -> 35.9 ms; two vortex instances of K = 131072, N = 2, 28 steps in two: 125 -> 115 ms.)
+// backward: 39.8 -> 35.0 ms; two vortex instances of K = 131072, N = 2, 28 steps in two: 125 -> 113 ms.)
 #pragma once
 
 namespace dg {
@@ -939,8 +939,8 @@ struct Adjoint {
     return t;
   }
 
-  // C_l of the solver's current q (device), optional gradient accumulation into lam.
-  cudaError_t lift(const Solver &s, double *lamacc, double wscale, double *cl_out, double *dcl_out) {
+  // C_l of q (device), optional gradient accumulation into lam.
+  cudaError_t lift(const Solver &s, const double *q, double *lamacc, double wscale, double *cl_out, double *dcl_out) {
     double elx, ely, delx, dely, iq;
     lift_dirs(elx, ely, delx, dely, iq);
     const int n = nbf();
@@ -949,7 +949,7 @@ struct Adjoint {
       *dcl_out = 0.0;
       return cudaSuccess;
     }
-    DG_DISPATCH(cfg.N, (cl_kernel<NN><<<(n + 127) / 128, 128, 0, s.stream>>>(s.d, s.d.q, parts, dparts, lamacc,
+    DG_DISPATCH(cfg.N, (cl_kernel<NN><<<(n + 127) / 128, 128, 0, s.stream>>>(s.d, q, parts, dparts, lamacc,
                                                                             wscale, iq, elx, ely, delx, dely)));
     det_sum_kernel<<<1, 256, 0, s.stream>>>(parts, n, scal);
     det_sum_kernel<<<1, 256, 0, s.stream>>>(dparts, n, scal + 1);
@@ -972,18 +972,22 @@ struct Adjoint {
     double acc = 0.0, dacc = 0.0;
     const int nl = (nsteps - 1) / C * C;  // first step of the last segment
     for (int n = 0; n < nsteps; n++) {
+      cudaError_t ce = cudaSuccess;
       if (n % C == 0)
-        if (cudaMemcpyAsync(ckpt + (size_t)(n / C) * nq(), s.d.q, nq() * 8, cudaMemcpyDeviceToDevice, s.stream) !=
-            cudaSuccess) { err = "checkpoint copy"; return -100; }
+        ce = cudaMemcpyAsync(ckpt + (size_t)(n / C) * nq(), s.d.q, nq() * 8, cudaMemcpyDeviceToDevice, s.stream);
+      if (n == nl && ce == cudaSuccess)
+        ce = cudaMemcpyAsync(seg, s.d.q, nq() * 8, cudaMemcpyDeviceToDevice, s.stream);
+      if (ce != cudaSuccess) { err = "checkpoint copy"; return -100; }
+      double *q = s.d.q;  // the state after the step
       if (n < nl) {
         s.enqueue_step(s.stream);
       } else {
-        step_stages(n - nl, s.stream);
-        s.enqueue_finalize(s.stream, true);
+        q = step_stages(n - nl, nsteps - nl, s.stream);
+        s.enqueue_finalize(s.stream, true, q);
       }
       if (cfg.app == 0 && n + 1 > nsteps - navg) {
         double cl, dcl;
-        if (lift(s, nullptr, 0.0, &cl, &dcl) != cudaSuccess) { err = "lift"; return -100; }
+        if (lift(s, q, nullptr, 0.0, &cl, &dcl) != cudaSuccess) { err = "lift"; return -100; }
         acc += cl;
         dacc += dcl;
       }
@@ -1011,24 +1015,35 @@ struct Adjoint {
     return 0;
   }
 
-  // The three stages of a step from the state in fwd, keeping q, W1, W2 in seg slot j.
-  void step_stages(int j, cudaStream_t st) {
-    Solver &s = *fwd;
+  // The three stages of step j of a segment of m steps.  Slot j of seg holds the step's q, and each stage
+  // writes the buffer that the next one reads: W1, W2, then the next slot's q (after the last step
+  // fwd's own q and W).  So the stages are kept without a copy, and the launches overlap as in any
+  // step: a forward run with no reverse sweep after it costs no more for them (40 steps in one
+  // segment, K = 2048 / 32768 at N = 3, 2.16 / 8.33 ms; with three copies per step 2.78 / 9.00 ms, without
+  // keeping them 2.16 / 8.36 ms).  Returns the new q.
+  double *step_stages(int j, int m, cudaStream_t st) {
     double *qj = seg + (size_t)(3 * j) * nq(), *w1 = qj + nq(), *w2 = w1 + nq();
-    cudaMemcpyAsync(qj, s.d.q, nq() * 8, cudaMemcpyDeviceToDevice, st);
-    DG_DISPATCH(cfg.N, {
-      launch_stage<NN>(s.d, 0, st);
-      cudaMemcpyAsync(w1, s.d.W, nq() * 8, cudaMemcpyDeviceToDevice, st);
-      launch_stage<NN>(s.d, 1, st);
-      cudaMemcpyAsync(w2, s.d.W, nq() * 8, cudaMemcpyDeviceToDevice, st);
-      launch_stage<NN>(s.d, 2, st);
-    });
+    Inst d = fwd->d;
+    d.q = d.W = qj;
+    d.Wo = w1;
+    DG_DISPATCH(cfg.N, launch_stage<NN>(d, 0, st));
+    d.W = w1;
+    d.Wo = w2;
+    DG_DISPATCH(cfg.N, launch_stage<NN>(d, 1, st));
+    d.W = w2;
+    if (j + 1 < m) {
+      d.qo = d.Wo = w2 + nq();
+    } else {
+      d.Wo = fwd->d.W;
+    }
+    DG_DISPATCH(cfg.N, launch_stage<NN>(d, 2, st));
+    return d.qo;
   }
 
-  // Re-run a step from the state in fwd (frozen dt), keeping its stages in seg slot j.
-  void recompute_step(int j, cudaStream_t st) {
+  // Re-run step j of a segment of m (frozen dt) from its slot's q, keeping its stages there.
+  void recompute_step(int j, int m, cudaStream_t st) {
     set_dt_kernel<<<1, 32, 0, st>>>(fwd->d.st, d_dts);
-    step_stages(j, st);
+    step_stages(j, m, st);
     finalize_kernel<<<1, 32, 0, st>>>(fwd->d.st, 1, nullptr, 0);
   }
 
@@ -1086,9 +1101,8 @@ struct Adjoint {
       cudaMemcpyAsync(s.d.st, &s0, sizeof(s0), cudaMemcpyHostToDevice, st);
       if (!kept) {
         seg_last = false;
-        cudaMemcpyAsync(s.d.q, ckpt + (size_t)sg * nq(), nq() * 8, cudaMemcpyDeviceToDevice, st);
-        cudaMemcpyAsync(s.d.W, s.d.q, nq() * 8, cudaMemcpyDeviceToDevice, st);
-        for (int n = n0; n < n1; n++) recompute_step(n - n0, st);
+        cudaMemcpyAsync(seg, ckpt + (size_t)sg * nq(), nq() * 8, cudaMemcpyDeviceToDevice, st);
+        for (int n = n0; n < n1; n++) recompute_step(n - n0, n1 - n0, st);
       }
       for (int n = n1 - 1; n >= n0; n--) {
         // objective term of q_{n+1}

@@ -278,7 +278,7 @@ __device__ __forceinline__ void stage_combine(const Inst &d, const int stage, co
   constexpr int Np = np_of(N);
   const Phys &P = d.P;
   const size_t off = ((size_t)(live ? e : 0) * Np + (active ? i : 0)) * 4;
-  double *wp = d.W + off;
+  double *wp = d.Wo + off;
   if (stage == 3) {
     if (live) {
       double *o = d.rhs_out + off;
@@ -296,7 +296,7 @@ __device__ __forceinline__ void stage_combine(const Inst &d, const int stage, co
     }
     return;
   }
-  double *qp = d.q + off;
+  const double *qp = d.q + off;
   double2 qa = make_double2(0.0, 0.0), qb = make_double2(0.0, 0.0);
   if (live) {
     if (qs) {
@@ -324,8 +324,9 @@ __device__ __forceinline__ void stage_combine(const Inst &d, const int stage, co
   n2 = fma(two_third, n2, third * qb.x);
   n3 = fma(two_third, n3, third * qb.y);
   if (live) {
-    st2(qp, n0, n1);
-    st2(qp + 2, n2, n3);
+    double *qo = d.qo + off;
+    st2(qo, n0, n1);
+    st2(qo + 2, n2, n3);
     st2(wp, n0, n1);
     st2(wp + 2, n2, n3);
     if (bad_density(n0)) atomicOr(&d.st->err, 1u);
@@ -1516,6 +1517,8 @@ int Solver::create(const Config &c, const Mesh &m, std::string &err) {
   const size_t nq = (size_t)K * Np * 4;
   d.q = (double *)dalloc(nq * 8);
   d.W = (double *)dalloc(nq * 8);
+  d.qo = d.q;
+  d.Wo = d.W;
   d.flux = (double *)dalloc((size_t)K * 3 * Nfp * 4 * 8);
   double *geo = (double *)dalloc((size_t)K * 16 * 8);
   d.geo = geo;
@@ -1582,13 +1585,15 @@ void Solver::enqueue_step(cudaStream_t s) {
   enqueue_finalize(s, true);
 }
 
-void Solver::enqueue_finalize(cudaStream_t s, bool pdl) {
+void Solver::enqueue_finalize(cudaStream_t s, bool pdl, double *q) {
   if (d.dt_mode == 0 && d.dt_est) {
+    Inst f = d;
+    if (q) f.q = q;
     // one block per SM at most, at least 32 estimates per block
     const int n = ((K + kDtCells - 1) / kDtCells) * np_of(cfg.N);
     const int g = std::max(1, std::min(sm_count > 0 ? sm_count : 1, (n + 31) / 32));
-    DG_DISPATCH(cfg.N, pdl ? launch_pdl(dt_finalize_kernel<NN>, dim3(g), dim3(256), 0, s, d)
-                           : (dt_finalize_kernel<NN><<<g, 256, 0, s>>>(d), void()));
+    DG_DISPATCH(cfg.N, pdl ? launch_pdl(dt_finalize_kernel<NN>, dim3(g), dim3(256), 0, s, f)
+                           : (dt_finalize_kernel<NN><<<g, 256, 0, s>>>(f), void()));
   } else if (pdl) {
     launch_pdl(finalize_kernel, dim3(1), dim3(32), 0, s, d.st, d.dt_mode, d.dt_hist, d.dt_hist_len);
   } else {

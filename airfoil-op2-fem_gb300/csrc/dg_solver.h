@@ -52,6 +52,7 @@ struct Inst {
   const double *bxy;
   const double *geo;
   double *q, *W, *flux;
+  double *qo, *Wo;  // where a stage writes q (the last one) and W: q and W themselves, but in the adjoint's kept steps
   double *rhs_out;
   StepState *st;
   double *dt_hist;
@@ -132,8 +133,8 @@ struct Solver {
   int set_dt_from_max(std::string &err);
   void enqueue_step(cudaStream_t s);
   // The step's last launch: t += dt, step += 1 and, with dt recomputed, the new dt (pdl: with
-  // programmatic dependence on the last element kernel).
-  void enqueue_finalize(cudaStream_t s, bool pdl);
+  // programmatic dependence on the last element kernel; q: the new state where it is not d.q).
+  void enqueue_finalize(cudaStream_t s, bool pdl, double *q = nullptr);
   int sm_count = 0;
   void enqueue_step_events(cudaStream_t s, cudaEvent_t *ev);
   int build_graph(std::string &err);
