@@ -2290,6 +2290,39 @@ extern "C" int dg_roe_flux_nodes(double gam, int form, int n, const double *qm, 
   return 0;
 }
 
+// dg_reciprocal_nodes (include/dg_gb300.h): the nodal fluxes' reciprocal beside the device's correctly rounded one.
+namespace dg {
+__global__ void reciprocal_kernel(int n, const double *x, double *seeded, double *rounded) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  seeded[k] = rcp_seeded(x[k]);
+  rounded[k] = rcp(x[k]);
+}
+}  // namespace dg
+
+extern "C" int dg_reciprocal_nodes(int n, const double *x, double *seeded, double *rounded) {
+  if (n <= 0 || n > (1 << 28) || !x || !seeded || !rounded) {
+    g_bstate_err = "bad arguments";
+    return DG_ERR_ARG;
+  }
+  const size_t m = (size_t)n;
+  double *d = nullptr;
+  cudaError_t ce = cudaMalloc(&d, m * 3 * sizeof(double));
+  if (ce == cudaSuccess) ce = cudaMemcpy(d, x, m * sizeof(double), cudaMemcpyHostToDevice);
+  if (ce == cudaSuccess) {
+    dg::reciprocal_kernel<<<(n + 255) / 256, 256>>>(n, d, d + m, d + 2 * m);
+    ce = cudaGetLastError();
+  }
+  if (ce == cudaSuccess) ce = cudaMemcpy(seeded, d + m, m * sizeof(double), cudaMemcpyDeviceToHost);
+  if (ce == cudaSuccess) ce = cudaMemcpy(rounded, d + 2 * m, m * sizeof(double), cudaMemcpyDeviceToHost);
+  if (d) cudaFree(d);
+  if (ce != cudaSuccess) {
+    g_bstate_err = std::string("dg_reciprocal_nodes: ") + cudaGetErrorString(ce);
+    return DG_ERR_CUDA;
+  }
+  return 0;
+}
+
 #include "dg_batch.cuh"
 #include "dg_adjoint.cuh"
 #include "dg_tangent.cuh"

@@ -353,6 +353,9 @@ int dg_roe_pair_flux(double gam, int n, const double *qm, const double *qp, cons
  * the general FP64 form, form 1 the rule (small-jump form where it applies).  Errors:
  * dg_boundary_state_error(). */
 int dg_roe_flux_nodes(double gam, int form, int n, const double *qm, const double *qp, const double *nrm, double *f2);
+/* The element kernels' reciprocal (seeded) of n values, and the device's correctly rounded one.  Errors:
+ * dg_boundary_state_error(). */
+int dg_reciprocal_nodes(int n, const double *x, double *seeded, double *rounded);
 /* Cell ranges of the step graph for solvers whose graph is built from now on: 0 automatic (the
  * default: ranges of at least 128 tiles of 32 cells, at most 4), 1 a single range (the seven
  * launches as one chain), 2..32 that many ranges (fewer if the mesh has fewer tiles). */
