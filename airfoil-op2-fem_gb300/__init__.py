@@ -130,6 +130,7 @@ def lib():
         "dg_elem_ws": (C.c_int, []),
         "dg_elem_variant": (C.c_int, []),
         "dg_tc_operator_digits": (C.c_int, [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
+        "dg_tc_operator_digits48": (C.c_int, [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
         "dg_tc_round": (C.c_int, [C.c_longlong, C.c_longlong, C.c_int, C.c_void_p]),
         "dg_set_face_block": (None, [C.c_int]),
         "dg_set_face_regs64": (None, [C.c_int]),

@@ -681,18 +681,24 @@ void dg_set_elem_blocks_per_sm(int blocks) { dg::set_elem_blocks_per_sm(blocks);
 int dg_elem_blocks_per_sm(void) { return dg::elem_blocks_per_sm(); }
 int dg_elem_ws(void) { return dg::elem_ws(); }
 
-int dg_tc_operator_digits(int N, int *dims, double *S, int *fexp, int *digits) {
+static int tc_tables(int N, int slots, int *dims, double *S, int *fexp, int *digits) {
   if (!dims) return fail(DG_ERR_ARG, "bad arguments");
   int d4[4], fe[2][32];
   std::vector<double> Sv;
   std::vector<int> dig;
   std::string err;
-  if (dg::tc_operator_tables(N, d4, Sv, fe, dig, err)) return fail(DG_ERR_ARG, err);
+  if (dg::tc_operator_tables(N, slots, d4, Sv, fe, dig, err)) return fail(DG_ERR_ARG, err);
   for (int k = 0; k < 4; k++) dims[k] = d4[k];
   if (S) std::copy(Sv.begin(), Sv.end(), S);
   if (fexp) std::copy(&fe[0][0], &fe[0][0] + 64, fexp);
   if (digits) std::copy(dig.begin(), dig.end(), digits);
   return 0;
+}
+int dg_tc_operator_digits(int N, int *dims, double *S, int *fexp, int *digits) {
+  return tc_tables(N, 32, dims, S, fexp, digits);
+}
+int dg_tc_operator_digits48(int N, int *dims, double *S, int *fexp, int *digits) {
+  return tc_tables(N, 48, dims, S, fexp, digits);
 }
 int dg_tc_round(long long th, long long tl, int sc, double *out) {
   if (!out || sc < -1022 || sc > 900) return fail(DG_ERR_ARG, "dg_tc_round: sc outside -1022..900");

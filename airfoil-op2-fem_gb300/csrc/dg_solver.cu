@@ -1326,10 +1326,14 @@ static void dense_rows(const Operators &o, std::vector<double> &A) {
 }
 
 // Host-only view of the tensor-core operator tables of order N (for tests): the parity
-// dimensions, the even/odd operator blocks S, the row exponents and the digits.
-int tc_operator_tables(int N, int dims[4], std::vector<double> &S, int fexp[2][kOzRows], std::vector<int> &dig,
-                       std::string &err) {
-  if (!oz_used(N, 1) || N > 5) { err = "no tensor-core tables of 32 slots at this order"; return -1; }
+// dimensions, the even/odd operator blocks S, the row exponents and the digits of the first `slots` of
+// the kOzSlots slots (32 hold all of them up to N = 5).
+int tc_operator_tables(int N, int slots, int dims[4], std::vector<double> &S, int fexp[2][kOzRows],
+                       std::vector<int> &dig, std::string &err) {
+  if (!oz_used(N, 1) || (slots < kOzSlots && N > 5) || slots > kOzSlots) {
+    err = "no tensor-core tables of " + std::to_string(slots) + " slots at this order";
+    return -1;
+  }
   Operators o;
   if (build_operators(N, o)) { err = "operator construction failed"; return -2; }
   std::vector<double> A;
@@ -1338,11 +1342,11 @@ int tc_operator_tables(int N, int dims[4], std::vector<double> &S, int fexp[2][k
   if (int rc = sym_build(o, A, t, err)) return rc;
   dims[0] = t.NUe; dims[1] = t.NUo; dims[2] = t.NRe; dims[3] = t.NRo;
   S = t.S;
-  std::vector<int> all;  // [2][7][kOzSlots][kOzRows], of which the first 32 slots hold all digits
+  std::vector<int> all;  // [2][7][kOzSlots][kOzRows]
   if (int rc = oz_digits(t.S, t.NUe, t.NUo, t.NRe, t.NRo, fexp, all, err)) return rc;
-  dig.resize((size_t)2 * 7 * 32 * kOzRows);
+  dig.resize((size_t)2 * 7 * slots * kOzRows);
   for (size_t b = 0; b < 2 * 7; b++)
-    std::copy_n(all.begin() + b * kOzSlots * kOzRows, 32 * kOzRows, dig.begin() + b * 32 * kOzRows);
+    std::copy_n(all.begin() + b * kOzSlots * kOzRows, slots * kOzRows, dig.begin() + b * slots * kOzRows);
   return 0;
 }
 

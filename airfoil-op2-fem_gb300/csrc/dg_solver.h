@@ -86,9 +86,9 @@ int elem_ws();
 void set_elem_blocks_per_sm(int b);
 int elem_blocks_per_sm();
 // Host-only: parity dimensions {NUe, NUo, NRe, NRo}, even/odd operator blocks, row exponents
-// [parity][32] and signed base-256 digits [parity][digit][slot 32][row 32] of the tensor-core
+// [parity][32] and signed base-256 digits [parity][digit][slot][row 32] of the tensor-core
 // contraction of order N.
-int tc_operator_tables(int N, int dims[4], std::vector<double> &S, int fexp[2][32], std::vector<int> &dig,
+int tc_operator_tables(int N, int slots, int dims[4], std::vector<double> &S, int fexp[2][32], std::vector<int> &dig,
                        std::string &err);
 // Host-only: (th 2^32 + tl) 2^sc rounded to the nearest double as the tensor-core contraction
 // rounds its level sums (valid for -1022 <= sc <= 900).
