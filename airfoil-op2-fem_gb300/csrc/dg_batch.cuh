@@ -197,6 +197,7 @@ struct Batch {
   cudaStream_t stream = nullptr;
   Inst *d_insts = nullptr;
   int4 *d_ftiles = nullptr, *d_etiles = nullptr;
+  size_t cap_ftiles = 0, cap_etiles = 0;  // their sizes, tiles
   int nft = 0, net = 0;
   int4 *d_fblocks = nullptr;  // blocks of batch_dt_finalize_kernel
   int nfb = 0;
@@ -274,7 +275,7 @@ struct Batch {
 
   // Element tiles (32 cells of one instance; with grouped launches small tiles where elem_small
   // chooses them for a mesh of all the order's cells), higher orders first; face tiles of ft nodes.
-  // The graphs hold the old tiles and go with them; on failure both stay as they were.
+  // The graphs hold the old tiles and go with them; where memory runs out both stay as they were.
   int build_tiles(int ft, bool grouped, std::string &err) {
     std::vector<int4> et, fts;
     const int fm = elem_form();
@@ -297,11 +298,11 @@ struct Batch {
       const int total = (d.nE + d.nB) * (d.N + 1);
       for (int f0 = 0; f0 < total; f0 += ft) fts.push_back(make_int4((int)k, f0, std::min(ft, total - f0), d.N));
     }
+    // buffers that are large enough are kept (the autotuner's candidates follow one another)
     int4 *df = nullptr, *de = nullptr;
-    cudaError_t ce = cudaMalloc(&df, sizeof(int4) * fts.size());
-    if (ce == cudaSuccess) ce = cudaMalloc(&de, sizeof(int4) * et.size());
-    if (ce == cudaSuccess) ce = cudaMemcpy(df, fts.data(), sizeof(int4) * fts.size(), cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess) ce = cudaMemcpy(de, et.data(), sizeof(int4) * et.size(), cudaMemcpyHostToDevice);
+    cudaError_t ce = cudaSuccess;
+    if (fts.size() > cap_ftiles) ce = cudaMalloc(&df, sizeof(int4) * fts.size());
+    if (ce == cudaSuccess && et.size() > cap_etiles) ce = cudaMalloc(&de, sizeof(int4) * et.size());
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(stream);  // steps in flight read the old tiles
     if (ce != cudaSuccess) {
       cudaGetLastError();
@@ -311,10 +312,23 @@ struct Batch {
       return -100;
     }
     drop_graphs();
-    if (d_ftiles) cudaFree(d_ftiles);
-    if (d_etiles) cudaFree(d_etiles);
-    d_ftiles = df;
-    d_etiles = de;
+    if (df) {
+      if (d_ftiles) cudaFree(d_ftiles);
+      d_ftiles = df;
+      cap_ftiles = fts.size();
+    }
+    if (de) {
+      if (d_etiles) cudaFree(d_etiles);
+      d_etiles = de;
+      cap_etiles = et.size();
+    }
+    ce = cudaMemcpy(d_ftiles, fts.data(), sizeof(int4) * fts.size(), cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) ce = cudaMemcpy(d_etiles, et.data(), sizeof(int4) * et.size(), cudaMemcpyHostToDevice);
+    if (ce != cudaSuccess) {
+      shape = BatchShape();  // no tiles: the next run makes its own
+      err = cudaGetErrorString(ce);
+      return -100;
+    }
     form = fm;
     std::copy(first, first + 7, ord_first);
     std::copy(count, count + 7, ord_count);
