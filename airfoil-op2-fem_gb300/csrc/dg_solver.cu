@@ -639,7 +639,7 @@ __global__ void __launch_bounds__(32 * np_of(N), MB) elem_kernel_sym(const Inst 
 
 // The same over tiles of elem_small_ct(N) cells (tensor-core forms, TC = 2; used as elem_small says):
 // elem_small_threads threads, of which CT Np hold a cell's node and every warp takes part in the
-// operand pre-pass and the contraction.  Compiled for 24 or 28 warps per SM, which at 128 to 256
+// operand pre-pass and the contraction.  Compiled for 24 or 28 warps per SM, which at 64 to 256
 // threads a block leaves 72 to 80 registers a thread (one block per SM: up to 127 registers and
 // fewer warps, K = 32768 N = 5 515 against 472 us per step; N = 2 at 24 / 28 warps 119.8 / 115.4 us).
 template <int N, bool PW>
